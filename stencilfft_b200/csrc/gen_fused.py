@@ -5,9 +5,17 @@ plan's `variant` picks one; "k3" marks the three-stage 512-thread pass of zm_fft
 for complex64 lines of 2^14 points ("k3p": its persistent form with asynchronous copies
 of the next line; "k3c": the forward y pass on buddy-line CTA pairs); "t" marks the
 persistent form of the fused pass whose next tile's first-phase points are staged in
-tensor memory (one CTA per SM).  Variant 0, the default, is
-the fastest one measured on B200 at the sizes the table was tuned on; zm_plan_autotune
-re-measures them for a plan."""
+tensor memory (one CTA per SM).  Variant 0, the default, is the axis pass of zm_axis.cuh
+(no instance here: zm_api.cu launches it) except for lines of 2^14 points at VEC = 64,
+M = 256, where it is the first entry of the list; the others are the
+alternatives that zm_plan_autotune measures for a plan."""
+
+
+def axis_default(lv, lm):
+    return (lv, lm) != (6, 8)
+
+
+
 VARIANTS = {
     "c64": {
         (4, 4): [(1, 32, 512)], (4, 5): [(1, 16, 512)], (4, 6): [(1, 8, 512), (1, 4, 256)],
@@ -39,7 +47,7 @@ VARIANTS = {
 # wait for those scattered reads: x 3.30 + y 3.70 = 6.97 ms per forward transform, against
 # 7.86 (two-line x tiles on clusters of four writing the 2-row interleave) and 8.51.
 FWD_OOP = {
-    "c64": {(6, 8): (7, 8, 3), (5, 8): (5, 5, 1), (6, 7): (2, 2, 1)},
+    "c64": {(6, 8): (7, 8, 3)},
     "c128": {(6, 8): (0, 3, 4)},
 }
 # Out-of-place 2D inverse configurations (caller workspace, default variant): y pass
@@ -72,6 +80,8 @@ for dt, table in VARIANTS.items():
              "    switch ((prm.g.logVEC << 16) | (prm.g.logM << 8) | prm.variant) {"]
         for (lv, lm), vs in table.items():
             for vi, v in enumerate(vs):
+                if vi == 0 and axis_default(lv, lm):
+                    continue
                 cl, tl, nt = v[:3]
                 pers = "true" if len(v) > 3 and v[3] == "p" else "false"
                 tms = ", true" if len(v) > 3 and v[3] == "t" else ""
@@ -98,6 +108,8 @@ for dt, table in VARIANTS.items():
                   "    switch ((logvec << 16) | (logm << 8) | variant) {"]
             for (lv, lm), vs in table.items():
                 for vi, v in enumerate(vs):
+                    if vi == 0 and axis_default(lv, lm):
+                        continue
                     cl, tl, nt = v[:3]
                     vec, n = 1 << lv, 1 << (lv + lm)
                     ept = tl * n // (cl * nt)

@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -160,7 +161,7 @@ static LineParams line_params(const zm_plan_s *p, int kind, const void *in, void
     lp.variant = p->variant;
     lp.permute_only = (p->flags & ZM_FLAG_PERMUTE_ONLY) ? 1 : 0;
     lp.err = p->dev_err;
-    // 2D transforms on the size-specialised passes keep the x -> y intermediate with
+    // 2D transforms on the size-specialised variants keep the x -> y intermediate with
     // groups of G x-frequency rows interleaved, G up to the tile's line count (at most
     // 4): the x pass then writes G * TL consecutive elements per line group and the y
     // pass reads its G lines as one contiguous run.  G <= VP keeps a group inside one
@@ -182,6 +183,7 @@ static LineParams line_params(const zm_plan_s *p, int kind, const void *in, void
 // in-place y pass rules out interleaves wider than its tile), or false.
 static bool fwd_oop_config(const zm_plan_s *p, int *vx, int *vy, int *lg, int *qint) {
     if (p->g.dim != 2 || (p->flags & ZM_FLAG_PERMUTE_ONLY) || p->nvariants == 0 || p->variant != 0) return false;
+    if (p->axis[0][0].ltl >= 0) return false;
     const int ok = p->dtype == ZM_C128 ? zm::fused_fwd_oop_c128(p->g.logVEC, p->g.logM, vx, vy, lg, qint)
                                        : zm::fused_fwd_oop_c64(p->g.logVEC, p->g.logM, vx, vy, lg, qint);
     if (!ok) return false;
@@ -192,6 +194,7 @@ static bool fwd_oop_config(const zm_plan_s *p, int *vx, int *vy, int *lg, int *q
 // work -> out), or false.
 static bool inv_oop_config(const zm_plan_s *p, int *vx, int *vy, int *lg, int *qint) {
     if (p->g.dim != 2 || (p->flags & ZM_FLAG_PERMUTE_ONLY) || p->nvariants == 0 || p->variant != 0) return false;
+    if (p->axis[0][0].ltl >= 0) return false;
     const int ok = p->dtype == ZM_C128 ? zm::fused_inv_oop_c128(p->g.logVEC, p->g.logM, vx, vy, lg, qint)
                                        : zm::fused_inv_oop_c64(p->g.logVEC, p->g.logM, vx, vy, lg, qint);
     if (!ok) return false;
@@ -202,7 +205,7 @@ static bool inv_oop_config(const zm_plan_s *p, int *vx, int *vy, int *lg, int *q
 // `variant` / `lg` >= 0 override the plan's tile shape and row interleave for this pass;
 // `qint` selects the y-position interleave of the intermediate.
 static int run_pass(const zm_plan_s *p, int kind, bool inv, const void *in, void *out, bool scale,
-                    double sre, double sim, cudaStream_t st, int variant = -1, int lg = -1, int qint = 0) {
+                    double sre, double sim, cudaStream_t st, int variant = -1, int lg = -1, int qint = 0, int oop = 0) {
     LineParams lp = line_params(p, kind, in, out);
     if (variant >= 0) lp.variant = variant;
     if (lg >= 0) lp.lg_inter = lg;
@@ -211,6 +214,21 @@ static int run_pass(const zm_plan_s *p, int kind, bool inv, const void *in, void
         lp.apply_scale = 1;
         lp.scale_re = sre;
         lp.scale_im = sim;
+    }
+    const int ax = kind == zm::PASS_X2 || kind == zm::PASS_X3 ? 0 : (kind == zm::PASS_Z3 ? 2 : 1);
+    if (p->axis[0][0].ltl >= 0 && p->variant == 0 && variant < 0) {
+        zm::AxisParams ap{};
+        ap.g = p->g;
+        ap.kind = kind;
+        ap.in = in;
+        ap.out = out;
+        ap.tw = p->twx;
+        ap.scale_re = lp.scale_re;
+        ap.scale_im = lp.scale_im;
+        ap.apply_scale = lp.apply_scale;
+        ap.m = p->axis[oop][ax];
+        cudaError_t ea = zm::launch_axis_pass(ap, p->dtype, inv, lp.nlines, st);
+        return ea == cudaSuccess ? ZM_OK : cuda_fail(ea, "axis pass launch");
     }
     cudaError_t e = zm::launch_line_pass(lp, p->dtype, inv, st);
     if (e != cudaSuccess) return cuda_fail(e, "line pass launch");
@@ -238,6 +256,12 @@ static int forward_impl(zm_plan p, const void *in, void *out, void *work, bool s
             // x pass in -> work, y pass work -> out (no in-place constraint on the tile)
             if ((rc = run_pass(p, zm::PASS_X2, false, in, work, false, 0, 0, st, vx, lg, qi))) return rc;
             return run_pass(p, zm::PASS_Y2, false, work, out, scale, sre, sim, st, vy, lg, qi);
+        }
+        if (work && p->axis[0][0].ltl >= 0 && p->variant == 0) {
+            if (overlap(work, in, F) || overlap(work, out, F))
+                return fail(ZM_ERR_INVALID_ARG, "work overlaps in/out");
+            if ((rc = run_pass(p, zm::PASS_X2, false, in, work, false, 0, 0, st, -1, -1, 0, 1))) return rc;
+            return run_pass(p, zm::PASS_Y2, false, work, out, scale, sre, sim, st, -1, -1, 0, 1);
         }
         // x pass: real layout -> REPACK layout (in -> out); y pass in place on out
         if ((rc = run_pass(p, zm::PASS_X2, false, in, out, false, 0, 0, st))) return rc;
@@ -338,11 +362,28 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     P->twN = P->twv = P->twm = P->twd = nullptr;
     P->dev_err = nullptr;
     P->own_work = nullptr;
+    P->twx = nullptr;
+    P->axis[0][0].ltl = -1;
+    std::vector<int64_t> exps;   // exponents of the axis pass' stage twiddles
+    int ltl = 0, lp = 0, le = 0;
+    if (!(flags & ZM_FLAG_PERMUTE_ONLY) && zm::axis_tile(g, dtype, total, &ltl, &lp, &le)) {
+        const int kinds[2][3] = {{zm::PASS_X2, zm::PASS_Y2, zm::PASS_Y2}, {zm::PASS_X3, zm::PASS_Y3, zm::PASS_Z3}};
+        // in place a y tile covers whole groups of interleaved rows: G <= TL
+        const int lg = ltl < 3 ? ltl : 3;
+        // with a workspace, one-line complex128 tiles write pairs of rows: whole sectors for
+        // the x pass (N = 8192 forward 1886 -> 1421 us, N = 4096 366 -> 285); four and eight
+        // rows are slower again (1428, 1522)
+        const int lgs[2] = {lg, dtype == ZM_C128 && ltl == 0 ? 1 : lg};
+        for (int o = 0; o < 2; o++)
+            for (int a = 0; a < dim; a++)
+                P->axis[o][a] = zm::axis_map(g, kinds[dim - 2][a], dtype, ltl, lp, le, lgs[o]);
+        zm::axis_twiddles(g, le, &exps);
+    }
     if (flags & ZM_FLAG_HOST_ONLY) {
         *plan = P;
         return ZM_OK;
     }
-    const int64_t entries = 2 * n + g.vec + g.m + 1;   // + one 16-byte slot for the error word
+    const int64_t entries = 2 * n + g.vec + g.m + 1 + (int64_t)exps.size();   // + one 16-byte slot for the error word
     std::vector<unsigned char> host((size_t)entries * 16);
     const long double pi = 3.141592653589793238462643383279502884L;
     auto put = [&](int64_t slot, int64_t m, int64_t len, bool fp64 = false) {   // w_len^m
@@ -362,6 +403,8 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     for (int64_t m = 0; m < n; m++) put(n + m, m, n, true);
     for (int64_t m = 0; m < g.vec; m++) put(2 * n + m, m, g.vec);
     for (int64_t m = 0; m < g.m; m++) put(2 * n + g.vec + m, m, g.m);
+    for (size_t i = 0; i < exps.size(); i++)
+        std::memcpy(&host[(size_t)(2 * n + g.vec + g.m + 1 + i) * 16], &host[(size_t)exps[i] * 16], 16);
     void *tables = nullptr;
     cudaError_t e = cudaMalloc(&tables, host.size());
     if (e != cudaSuccess) {
@@ -380,6 +423,7 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     P->twv = tb + (size_t)2 * n * 16;
     P->twm = tb + (size_t)(2 * n + g.vec) * 16;
     P->dev_err = reinterpret_cast<int *>(tb + (size_t)(2 * n + g.vec + g.m) * 16);   // zeroed by the upload
+    P->twx = tb + (size_t)(2 * n + g.vec + g.m + 1) * 16;
     if (flags & ZM_FLAG_OWN_WORKSPACE) {
         e = cudaMalloc(&P->own_work, (size_t)P->total * P->elem_bytes);
         if (e != cudaSuccess) {

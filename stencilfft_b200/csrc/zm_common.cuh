@@ -7,6 +7,7 @@
 #include "zm_plan.h"
 
 #define ZM_DEV __device__ __forceinline__
+#define ZM_HD __host__ __device__ __forceinline__
 
 namespace zm {
 
@@ -175,9 +176,18 @@ struct k32 {
                                     0.38268343236508977173,    // cos(3pi/8)
                                     0.19509032201612826785,    // cos(7pi/16)
                                     0.0};
+    // what rounding them to double leaves
+    static constexpr double lo[9] = {0.0, 1.8546939997825006e-17, 1.7645047084336677e-17, 1.4073856984728024e-18,
+                                     -4.833646656726457e-17, 4.709410940561677e-17, -1.0050772696461588e-17,
+                                     -7.991079068461731e-18, 0.0};
 };
 
-template <int R, int K, int DIR, typename T> ZM_DEV cpx<T> cmul_const(cpx<T> v) {
+// COMP: constants as hi + lo of the working precision, every product fused: 1 the 45 degree
+// ones (every third multiplication, and the cheapest to do: three operations per component
+// instead of two), 2 also those of a 32-point codelet's last level, 3 all.  A rounded
+// constant is the same factor in every transform, so its error adds up coherently, twice in
+// a round trip.
+template <int R, int K, int DIR, typename T, int COMP = 0> ZM_DEV cpx<T> cmul_const(cpx<T> v) {
     constexpr int k = ((K % R) + R) % R;
     constexpr int kc = k * (32 / R);          // position on the 32-point circle (R <= 32)
     static_assert(32 % R == 0, "radix must divide 32");
@@ -197,24 +207,38 @@ template <int R, int K, int DIR, typename T> ZM_DEV cpx<T> cmul_const(cpx<T> v) 
         constexpr double sgn = kc >= 16 ? -1.0 : 1.0;    // add pi
         constexpr double cc = sgn * c0, ss = sgn * s0 * (DIR < 0 ? -1.0 : 1.0);
         const T c = (T)cc, s = (T)ss;
+        if constexpr (COMP >= 3 || (COMP == 2 && R == 32) || (COMP >= 1 && q % 8 == 4)) {
+            constexpr double lc0 = q <= 8 ? k32::lo[q] : -k32::lo[16 - q], ls0 = q <= 8 ? k32::lo[8 - q] : k32::lo[q - 8];
+            constexpr double lcc = sgn * lc0, lss = sgn * ls0 * (DIR < 0 ? -1.0 : 1.0);
+            const T cl = sizeof(T) == 4 ? (T)(cc - (double)(T)cc) : (T)lcc;
+            const T sl = sizeof(T) == 4 ? (T)(ss - (double)(T)ss) : (T)lss;
+            if constexpr (q == 4 || q == 12) {       // |c| = |s|: one product per component
+                constexpr bool same = (cc > 0) == (ss > 0);
+                const T re = same ? v.x - v.y : v.x + v.y, im = same ? v.x + v.y : v.y - v.x;
+                return {fma(re, c, re * cl), fma(im, c, im * cl)};
+            }
+            const T re = fma(v.x, c, fma(-v.y, s, fma(v.x, cl, -v.y * sl)));
+            const T im = fma(v.x, s, fma(v.y, c, fma(v.x, sl, v.y * cl)));
+            return {re, im};
+        }
         return {v.x * c - v.y * s, v.x * s + v.y * c};
     }
 }
 
-template <int H, int R, int DIR, typename T, int K = 0> struct combine {
+template <int H, int R, int DIR, typename T, int K = 0, int COMP = 0> struct combine {
     ZM_DEV static void run(cpx<T> *v, const cpx<T> *e, const cpx<T> *o) {
         if constexpr (K < H) {
-            cpx<T> t = cmul_const<R, K, DIR>(o[K]);
+            cpx<T> t = cmul_const<R, K, DIR, T, COMP>(o[K]);
             v[K] = cadd(e[K], t);
             v[K + H] = csub(e[K], t);
-            combine<H, R, DIR, T, K + 1>::run(v, e, o);
+            combine<H, R, DIR, T, K + 1, COMP>::run(v, e, o);
         }
     }
 };
 
 // In-register DFT of R points, natural order in and out (radix-2 DIT recursion
-// with the trivial rotations folded away).
-template <int R, int DIR, typename T> ZM_DEV void dft(cpx<T> *v) {
+// with the trivial rotations folded away).  COMP: compensated constants.
+template <int R, int DIR, typename T, int COMP = 0> ZM_DEV void dft(cpx<T> *v) {
     if constexpr (R == 1) {
         return;
     } else if constexpr (R == 2) {
@@ -226,9 +250,9 @@ template <int R, int DIR, typename T> ZM_DEV void dft(cpx<T> *v) {
         cpx<T> e[H], o[H];
 #pragma unroll
         for (int i = 0; i < H; i++) { e[i] = v[2 * i]; o[i] = v[2 * i + 1]; }
-        dft<H, DIR, T>(e);
-        dft<H, DIR, T>(o);
-        combine<H, R, DIR, T>::run(v, e, o);
+        dft<H, DIR, T, COMP>(e);
+        dft<H, DIR, T, COMP>(o);
+        combine<H, R, DIR, T, 0, COMP>::run(v, e, o);
     }
 }
 
@@ -236,7 +260,7 @@ template <int R, int DIR, typename T> ZM_DEV void dft(cpx<T> *v) {
 ZM_DEV int64_t pack_pos(int64_t i, int logB, int64_t B, int logVEC) {   // block_cyclic_to_packed
     return ((i & (B - 1)) << logVEC) + (i >> logB);
 }
-ZM_DEV int64_t unpack_pos(int64_t q, int64_t VEC, int logVEC, int logB) {  // inverse of pack_pos
+ZM_HD int64_t unpack_pos(int64_t q, int64_t VEC, int logVEC, int logB) {  // inverse of pack_pos
     return ((q & (VEC - 1)) << logB) + (q >> logVEC);
 }
 

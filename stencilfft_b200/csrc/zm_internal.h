@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "zm_plan.h"
 
 namespace zm {
@@ -39,6 +41,17 @@ int fused_fwd_oop_c128(int logvec, int logm, int *vx, int *vy, int *lg, int *qin
 // the same for the out-of-place 2D inverse (y pass in -> work, x pass work -> out)
 int fused_inv_oop_c64(int logvec, int logm, int *vx, int *vy, int *lg, int *qint);
 int fused_inv_oop_c128(int logvec, int logm, int *vx, int *vy, int *lg, int *qint);
+
+// zm_axis.cu: the axis pass sized by N alone
+bool axis_tile(const Geom &g, int dtype, int64_t total, int *ltl, int *lp, int *le);
+AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, int le, int lg);
+int64_t axis_twiddles(const Geom &g, int le, std::vector<int64_t> *exps);
+cudaError_t launch_axis_pass(const AxisParams &p, int dtype, bool inv, int64_t nlines, cudaStream_t st);
+// zm_axis_<dtype>_<dir>.cu
+cudaError_t launch_axis_c64_fwd(const AxisParams &p, int64_t nlines, cudaStream_t st);
+cudaError_t launch_axis_c64_inv(const AxisParams &p, int64_t nlines, cudaStream_t st);
+cudaError_t launch_axis_c128_fwd(const AxisParams &p, int64_t nlines, cudaStream_t st);
+cudaError_t launch_axis_c128_inv(const AxisParams &p, int64_t nlines, cudaStream_t st);
 
 // zm_stencil.cu
 enum StencilOp : int { ST_LAPLACE = 0, ST_DX = 1, ST_DY = 2, ST_ALL = 3 };

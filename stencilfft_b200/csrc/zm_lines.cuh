@@ -28,7 +28,7 @@ struct LineAddr {
     int f_lg;
 };
 
-ZM_DEV LineAddr line_addr(const Geom &g, int kind, int64_t l, int lg = 0, bool qint = false) {
+ZM_HD LineAddr line_addr(const Geom &g, int kind, int64_t l, int lg = 0, bool qint = false) {
     LineAddr a;
     const int64_t L = g.L, P = g.p, LL = L * L, LLL = LL * L;
     a.a_pos = 1;

@@ -49,6 +49,31 @@ struct LineParams {
     int rad_vec[8], rad_m[8];
 };
 
+// The layout of one axis pass as weights per bit (zm_axis.cuh): a tile of 2^ltl lines x N
+// points, 2^lp points per thread, digits of at most 2^le points.
+struct AxisMap {
+    int ltl, lp, le;   // ltl = -1: no tile of this pass
+    int lg;            // log2 of the row interleave of the 2D intermediate
+    // vector side, in address order: weights of the thread bits, then of the register bits
+    // (complex64: register bit 0 is the lowest address bit); addresses and tile slots
+    int va[16], vs[16];
+    // frequency side: the index bits outside the edge stage's digit, thread bits then unit
+    // bits (addresses, tile slots), and the digit's address weights
+    int fa[16], fs[16], fr[8];
+};
+
+// Parameters of one launch of the axis pass sized by N alone.
+struct AxisParams {
+    Geom g;
+    int kind;
+    const void *in;
+    void *out;
+    const void *tw;    // stage twiddles of (N, le)
+    double scale_re, scale_im;
+    int apply_scale;
+    AxisMap m;
+};
+
 }  // namespace zm
 
 struct zm_plan_s {
@@ -67,5 +92,9 @@ struct zm_plan_s {
     int variant;      // tile-shape variant of the size-specialised kernel
     int nvariants;    // variants available for (VEC, M, dtype); 0 = runtime-sized kernel only
     int *dev_err;     // device error word (bounded waits that gave up), inside the tables allocation
+    // the passes x, y, z on the kernel sized by N alone: [0] in place, [1] 2D forward with
+    // a workspace (its own row interleave)
+    zm::AxisMap axis[2][3];
+    void *twx;        // its stage twiddles (inside the tables allocation)
     void *own_work;   // ZM_FLAG_OWN_WORKSPACE: one field, used by transforms called with work = NULL
 };
