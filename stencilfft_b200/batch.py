@@ -19,6 +19,7 @@ class Batch:
         if not (len(ns) == len(bs) == len(ps)) or len(ns) == 0:
             raise ValueError("ns, bs and ps must be non-empty and of equal length")
         self.dtype = _DT[dtype]
+        self._dt = None           # the torch dtype, once torch is needed
         arr = ctypes.c_int64 * len(ns)
         h = ctypes.c_void_p()
         check(lib().zm_batch_create(ctypes.byref(h), len(ns), arr(*ns), arr(*bs), arr(*ps), self.dtype),
@@ -50,6 +51,10 @@ class Batch:
     def _check(self, t, name):
         if t is None:
             raise ValueError(f"{name} is required")
+        if self._dt is None:
+            self._dt = self.torch_dtype
+        if t.dtype is self._dt and t.numel() >= self.total and t.is_cuda and t.is_contiguous():
+            return
         if t.dtype != self.torch_dtype or t.numel() < self.total or not t.is_cuda or not t.is_contiguous():
             raise ValueError(f"{name}: expected a contiguous CUDA {self.torch_dtype} tensor of >= "
                              f"{self.total} elements")
