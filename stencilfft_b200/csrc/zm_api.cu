@@ -385,24 +385,18 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     }
     const int64_t entries = 2 * n + g.vec + g.m + 1 + (int64_t)exps.size();   // + one 16-byte slot for the error word
     std::vector<unsigned char> host((size_t)entries * 16);
-    const long double pi = 3.141592653589793238462643383279502884L;
-    auto put = [&](int64_t slot, int64_t m, int64_t len, bool fp64 = false) {   // w_len^m
-        const long double th = -2.0L * pi * (long double)m / (long double)len;
-        const double c = (double)cosl(th), s = (double)sinl(th);
-        if (dtype == ZM_C128 || fp64) {
-            double *d = reinterpret_cast<double *>(host.data()) + 2 * slot;
-            d[0] = c; d[1] = s;
-        } else {
-            float *f = reinterpret_cast<float *>(host.data()) + 4 * slot;
-            const float ch = (float)c, sh = (float)s;
-            f[0] = ch; f[1] = sh;
-            f[2] = (float)(c - (double)ch); f[3] = (float)(s - (double)sh);
-        }
+    // w_N^m once; the other tables are subsets of it (VEC, M divide N, all powers of two)
+    std::vector<double> w((size_t)(2 * n));
+    zm::unit_roots(n, w.data());
+    auto put = [&](int64_t slot, int64_t m, bool fp64 = false) {
+        unsigned char *at = host.data() + (size_t)slot * 16;
+        if (fp64) std::memcpy(at, &w[2 * m], 16);
+        else zm::twiddle_store(dtype, w[2 * m], w[2 * m + 1], at);
     };
-    for (int64_t m = 0; m < n; m++) put(m, m, n);
-    for (int64_t m = 0; m < n; m++) put(n + m, m, n, true);
-    for (int64_t m = 0; m < g.vec; m++) put(2 * n + m, m, g.vec);
-    for (int64_t m = 0; m < g.m; m++) put(2 * n + g.vec + m, m, g.m);
+    for (int64_t m = 0; m < n; m++) put(m, m);
+    for (int64_t m = 0; m < n; m++) put(n + m, m, true);
+    for (int64_t m = 0; m < g.vec; m++) put(2 * n + m, m * g.m);
+    for (int64_t m = 0; m < g.m; m++) put(2 * n + g.vec + m, m * g.vec);
     for (size_t i = 0; i < exps.size(); i++)
         std::memcpy(&host[(size_t)(2 * n + g.vec + g.m + 1 + i) * 16], &host[(size_t)exps[i] * 16], 16);
     void *tables = nullptr;

@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "zm_axis.cuh"
 #include "zm_axis_tiles.h"
@@ -140,6 +141,33 @@ int64_t axis_twiddles(const Geom &g, int le, std::vector<int64_t> *exps) {
                 exps->push_back(((k * v) << (ln - lr - sh)) & (g.n - 1));
     }
     return (int64_t)exps->size();
+}
+
+void unit_roots(int64_t n, double *w) {
+    const long double pi = 3.141592653589793238462643383279502884L;
+    for (int64_t m = 0; m < n; m++) {
+        const long double th = -2.0L * pi * (long double)m / (long double)n;
+        w[2 * m] = (double)cosl(th);
+        w[2 * m + 1] = (double)sinl(th);
+    }
+}
+
+void twiddle_store(int dtype, double c, double s, void *at) {
+    if (dtype == 0) {
+        const double d[2] = {c, s};
+        memcpy(at, d, 16);
+    } else {
+        const float ch = (float)c, sh = (float)s;
+        const float f[4] = {ch, sh, (float)(c - (double)ch), (float)(s - (double)sh)};
+        memcpy(at, f, 16);
+    }
+}
+
+void twiddle_entries(int64_t n, int dtype, const std::vector<int64_t> &exps, void *out) {
+    std::vector<double> w((size_t)(2 * n));
+    unit_roots(n, w.data());
+    for (size_t i = 0; i < exps.size(); i++)
+        twiddle_store(dtype, w[2 * exps[i]], w[2 * exps[i] + 1], static_cast<unsigned char *>(out) + 16 * i);
 }
 
 cudaError_t launch_axis_pass(const AxisParams &p, int dtype, bool inv, int64_t nlines, cudaStream_t st) {

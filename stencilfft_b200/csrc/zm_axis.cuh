@@ -59,27 +59,39 @@ template <typename T, int LN, int LTL, int LP, int LE> struct AxisCfg {
     static constexpr int MINB = MINB0 < 1 ? 1 : (MINB0 > 16 ? 16 : MINB0);
 };
 
-// sums over the set bits of tid of two weight lists
-template <int NB> ZM_DEV void axis_bits(int tid, const int *wa, const int *ws, int &a, int &s) {
-    a = 0;
-    s = 0;
-#pragma unroll
-    for (int b = 0; b < NB; b++) {
-        const int m = (tid >> b) & 1;
-        a += m * wa[b];
-        s += m * ws[b];
-    }
-}
-// offset of register r: the sum of the weights w[0 ..] over its set bits
-template <int NB> ZM_DEV int axis_reg(int r, const int *w) {
+// The weight tables as the kernel sees them: launch parameters, or a table in global memory
+// (batches, one per field layout).
+struct AxisParamMap {
+    static constexpr bool CONST_IN = true;    // the input is constant while the kernel runs
+    static constexpr int COMP64 = 2;          // compensated codelet constants in complex64 (dft)
+    const AxisMap &m;
+    ZM_DEV int va(int i) const { return m.va[i]; }
+    ZM_DEV int vs(int i) const { return m.vs[i]; }
+    ZM_DEV int fa(int i) const { return m.fa[i]; }
+    ZM_DEV int fs(int i) const { return m.fs[i]; }
+    ZM_DEV int fr(int i) const { return m.fr[i]; }
+};
+struct AxisGlobalMap {
+    static constexpr bool CONST_IN = false;   // an earlier step of the launch may have written it
+    static constexpr int COMP64 = 3;          // phi of 256 x 256^2: 1.86e-7 of FP64 with 2, 1.76e-7 with 3, 0.5 % slower
+    const AxisMap *m;
+    ZM_DEV int va(int i) const { return __ldg(m->va + i); }
+    ZM_DEV int vs(int i) const { return __ldg(m->vs + i); }
+    ZM_DEV int fa(int i) const { return __ldg(m->fa + i); }
+    ZM_DEV int fs(int i) const { return __ldg(m->fs + i); }
+    ZM_DEV int fr(int i) const { return __ldg(m->fr + i); }
+};
+
+// sum of the weights w(0 .. NB - 1) over the set bits of x (a constant, once unrolled, for
+// the registers of a thread)
+template <int NB, typename W> ZM_DEV int axis_bits(int x, W &&w) {
     int o = 0;
 #pragma unroll
-    for (int b = 0; b < NB; b++)
-        if (r >> b & 1) o += w[b];
+    for (int b = 0; b < NB; b++) o += (x >> b & 1) * w(b);
     return o;
 }
 
-template <typename T, int LN, int LTL, int LP, int LE, bool INV> struct AxisPass {
+template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = AxisParamMap> struct AxisPass {
     using C = cpx<T>;
     using CF = AxisCfg<T, LN, LTL, LP, LE>;
     static constexpr int NT = CF::NT, LNT = CF::LNT, NST = CF::NST, EPT = 1 << LP;
@@ -88,130 +100,142 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV> struct AxisPass
     // Round trip against FP64, without and with: 3D N = 256 c64 2.8e-7 / 2.4e-7 (at every
     // constant 2.2e-7), N = 1024 (32-point digits) 2.8e-7 / 2.2e-7, 3D N = 512 3.3e-7 /
     // 2.6e-7; 3D N = 256 c128 5.4e-16 / 4.2e-16; times within 1 % of each other.
-    static constexpr int COMP = sizeof(T) == 4 ? 2 : 1;
+    static constexpr int COMP = sizeof(T) == 4 ? MAP::COMP64 : 1;
 
     // global vector side <-> tile, in address order: thread bits first; complex64 keeps the
     // lowest address bit in the registers (16-byte accesses)
-    static ZM_DEV void load_vec(C *S, const C *in, const AxisMap &m, int tid) {
-        int a0, s0;
-        axis_bits<LNT>(tid, m.va, m.vs, a0, s0);
+    static ZM_DEV void load_vec(C *S, const C *in, const MAP &m, int tid) {
+        in += axis_bits<LNT>(tid, [&](int b) { return m.va(b); });
+        S += axis_bits<LNT>(tid, [&](int b) { return m.vs(b); });
+        auto ra = [&](int r) { return axis_bits<LP>(r, [&](int b) { return m.va(LNT + b); }); };
+        auto rs = [&](int r) { return axis_bits<LP>(r, [&](int b) { return m.vs(LNT + b); }); };
         C v[EPT];
         if constexpr (sizeof(T) == 4) {
 #pragma unroll
             for (int r = 0; r < EPT; r += 2) {
-                const float4 q = __ldg(reinterpret_cast<const float4 *>(in + a0 + axis_reg<LP>(r, m.va + LNT)));
+                const float4 *g = reinterpret_cast<const float4 *>(in + ra(r));
+                const float4 q = MAP::CONST_IN ? __ldg(g) : *g;
                 v[r] = {q.x, q.y};
                 v[r + 1] = {q.z, q.w};
             }
         } else {
 #pragma unroll
-            for (int r = 0; r < EPT; r++) v[r] = ldg(in + a0 + axis_reg<LP>(r, m.va + LNT));
+            for (int r = 0; r < EPT; r++) v[r] = MAP::CONST_IN ? ldg(in + ra(r)) : in[ra(r)];
         }
 #pragma unroll
-        for (int r = 0; r < EPT; r++) S[s0 + axis_reg<LP>(r, m.vs + LNT)] = v[r];
+        for (int r = 0; r < EPT; r++) S[rs(r)] = v[r];
     }
-    static ZM_DEV void store_vec(const C *S, C *out, const AxisMap &m, int tid, bool scl, T sr, T si) {
-        int a0, s0;
-        axis_bits<LNT>(tid, m.va, m.vs, a0, s0);
+    static ZM_DEV void store_vec(const C *S, C *out, const MAP &m, int tid, bool scl, T sr, T si) {
+        out += axis_bits<LNT>(tid, [&](int b) { return m.va(b); });
+        S += axis_bits<LNT>(tid, [&](int b) { return m.vs(b); });
+        auto ra = [&](int r) { return axis_bits<LP>(r, [&](int b) { return m.va(LNT + b); }); };
+        auto rs = [&](int r) { return axis_bits<LP>(r, [&](int b) { return m.vs(LNT + b); }); };
         constexpr int ST = sizeof(T) == 4 ? 2 : 1;
 #pragma unroll
         for (int r = 0; r < EPT; r += ST) {
             C v[ST];
 #pragma unroll
             for (int q = 0; q < ST; q++) {
-                v[q] = S[s0 + axis_reg<LP>(r + q, m.vs + LNT)];
+                v[q] = S[rs(r + q)];
                 if (scl) v[q] = {sr * v[q].x - si * v[q].y, sr * v[q].y + si * v[q].x};
             }
-            C *o = out + a0 + axis_reg<LP>(r, m.va + LNT);
-            if constexpr (ST == 2) *reinterpret_cast<float4 *>(o) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-            else *o = v[0];
+            if constexpr (ST == 2)
+                *reinterpret_cast<float4 *>(out + ra(r)) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+            else out[ra(r)] = v[0];
         }
     }
 
-    // stage s on the units of this thread; the stage next to the frequency side (the last
-    // forward, the first inverse) takes its units in frequency-side order and reads or
-    // writes global memory at `gm`
-    template <int s> static ZM_DEV void stage(C *S, C *gm, const AxisParams &p, int tid, bool scl, T sr, T si) {
-        constexpr int lr = axis_lr(LN, LE, s), sh = axis_sh(LN, LE, s), shp = sh + LTL;
-        constexpr int R = 1 << lr, LU = LP - lr;
-        constexpr bool EDGE = s == NST - 1;
-        if constexpr (EDGE) {
-            int fa0, fs0;
-            axis_bits<LNT>(tid, p.m.fa, p.m.fs, fa0, fs0);
+    // The stage next to the frequency side (the last one forward, the first inverse): units
+    // in frequency-side order, global memory at `gm` on that side.
+    static ZM_DEV void edge_stage(C *S, C *gm, const MAP &m, int tid, bool scl, T sr, T si) {
+        constexpr int lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, LU = LP - lr;
+        gm += axis_bits<LNT>(tid, [&](int b) { return m.fa(b); });
+        S += axis_bits<LNT>(tid, [&](int b) { return m.fs(b); });
+        auto ga = [&](int r) { return axis_bits<lr>(r, [&](int b) { return m.fr(b); }); };
 #pragma unroll
-            for (int u = 0; u < 1 << LU; u++) {
-                C x[R];
-                const int slot = fs0 + axis_reg<LU>(u, p.m.fs + LNT);
-                C *g = gm + fa0 + axis_reg<LU>(u, p.m.fa + LNT);
+        for (int u = 0; u < 1 << LU; u++) {
+            C x[R];
+            C *s = S + axis_bits<LU>(u, [&](int b) { return m.fs(LNT + b); });
+            C *g = gm + axis_bits<LU>(u, [&](int b) { return m.fa(LNT + b); });
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    if constexpr (INV) x[r] = ldg(g + axis_reg<lr>(r, p.m.fr));
-                    else x[r] = S[slot + axis_slot(r << shp)];
-                }
-                dft<R, DIR, T, COMP>(x);
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    if constexpr (INV) {
-                        S[slot + axis_slot(r << shp)] = x[r];
-                    } else {
-                        if (scl) x[r] = {x[r].x * sr - x[r].y * si, x[r].x * si + x[r].y * sr};
-                        g[axis_reg<lr>(r, p.m.fr)] = x[r];
-                    }
-                }
+            for (int r = 0; r < R; r++) {
+                if constexpr (INV) x[r] = MAP::CONST_IN ? ldg(g + ga(r)) : g[ga(r)];
+                else x[r] = s[axis_slot(r << LTL)];
             }
-        } else {
-            // thread -> (low line bits, v, index bits above the digit); the units of one `h`
-            // differ in the highest line bits only
-            constexpr int LUT = LTL < LU ? LTL : LU, LT0 = LTL - LUT, HI = 1 << (LU - LUT), LO = 1 << LUT;
-            const tw<T> *tb = reinterpret_cast<const tw<T> *>(p.tw) + axis_tw(LN, LE, s);
+            dft<R, DIR, T, COMP>(x);
 #pragma unroll
-            for (int h = 0; h < HI; h++) {
-                const int U = tid + h * NT;
-                const int iv = U >> LT0;                       // (bits above the digit, v)
-                const int v = iv & ((1 << sh) - 1);
-                const int i = ((iv >> sh) << (sh + lr)) | v;
-                const int slot = axis_slot((i << LTL) | (U & ((1 << LT0) - 1)));
-                C x[LO][R];
-#pragma unroll
-                for (int q = 0; q < LO; q++) {
-#pragma unroll
-                    for (int r = 0; r < R; r++) x[q][r] = S[slot + axis_slot(q << LT0 | r << shp)];
-                }
+            for (int r = 0; r < R; r++) {
                 if constexpr (INV) {
-#pragma unroll
-                    for (int r = 1; r < R; r++) {
-                        const tw<T> w = ldtw(tb, (r << sh) + v);
-#pragma unroll
-                        for (int q = 0; q < LO; q++) x[q][r] = twmul<true>(x[q][r], w);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < LO; q++) dft<R, DIR, T, COMP>(x[q]);
-                if constexpr (!INV) {
-#pragma unroll
-                    for (int r = 1; r < R; r++) {
-                        const tw<T> w = ldtw(tb, (r << sh) + v);
-#pragma unroll
-                        for (int q = 0; q < LO; q++) x[q][r] = twmul<false>(x[q][r], w);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < LO; q++) {
-#pragma unroll
-                    for (int r = 0; r < R; r++) S[slot + axis_slot(q << LT0 | r << shp)] = x[q][r];
+                    s[axis_slot(r << LTL)] = x[r];
+                } else {
+                    if (scl) x[r] = {x[r].x * sr - x[r].y * si, x[r].x * si + x[r].y * sr};
+                    g[ga(r)] = x[r];
                 }
             }
         }
     }
-    template <int s> static ZM_DEV void forward_from(C *S, C *gm, const AxisParams &p, int tid, bool scl, T sr, T si) {
-        __syncthreads();
-        stage<s>(S, gm, p, tid, scl, sr, si);
-        if constexpr (s + 1 < NST) forward_from<s + 1>(S, gm, p, tid, scl, sr, si);
+    // An inner stage: thread -> (low line bits, v, index bits above the digit); the units of
+    // one `h` differ in the highest line bits only and share their twiddles.
+    template <int s> static ZM_DEV void inner_stage(C *S, const tw<T> *tb, int tid) {
+        constexpr int lr = axis_lr(LN, LE, s), sh = axis_sh(LN, LE, s), shp = sh + LTL, R = 1 << lr, LU = LP - lr;
+        constexpr int LUT = LTL < LU ? LTL : LU, LT0 = LTL - LUT, HI = 1 << (LU - LUT), LO = 1 << LUT;
+        tb += axis_tw(LN, LE, s);
+#pragma unroll
+        for (int h = 0; h < HI; h++) {
+            const int U = tid + h * NT;
+            const int iv = U >> LT0;                       // (bits above the digit, v)
+            const int v = iv & ((1 << sh) - 1);
+            const int i = ((iv >> sh) << (sh + lr)) | v;
+            const int slot = axis_slot((i << LTL) | (U & ((1 << LT0) - 1)));
+            C x[LO][R];
+#pragma unroll
+            for (int q = 0; q < LO; q++) {
+#pragma unroll
+                for (int r = 0; r < R; r++) x[q][r] = S[slot + axis_slot(q << LT0 | r << shp)];
+            }
+            auto twiddle = [&]() {
+#pragma unroll
+                for (int r = 1; r < R; r++) {
+                    const tw<T> w = ldtw(tb, (r << sh) + v);
+#pragma unroll
+                    for (int q = 0; q < LO; q++) x[q][r] = twmul<INV>(x[q][r], w);
+                }
+            };
+            if constexpr (INV) twiddle();
+#pragma unroll
+            for (int q = 0; q < LO; q++) dft<R, DIR, T, COMP>(x[q]);
+            if constexpr (!INV) twiddle();
+#pragma unroll
+            for (int q = 0; q < LO; q++) {
+#pragma unroll
+                for (int r = 0; r < R; r++) S[slot + axis_slot(q << LT0 | r << shp)] = x[q][r];
+            }
+        }
     }
-    template <int s> static ZM_DEV void inverse_from(C *S, C *gm, const AxisParams &p, int tid) {
-        stage<s>(S, gm, p, tid, false, T(1), T(0));
+    // stages s .. NST - 2 forward, s .. 0 inverse, a barrier before / after each
+    template <int s> static ZM_DEV void inner_stages(C *S, const tw<T> *tb, int tid) {
+        if constexpr (s >= 0 && s < NST - 1) {
+            if constexpr (!INV) __syncthreads();
+            inner_stage<s>(S, tb, tid);
+            if constexpr (INV) __syncthreads();
+            inner_stages<(INV ? s - 1 : s + 1)>(S, tb, tid);
+        }
+    }
+    // vector side -> frequency side
+    static ZM_DEV void forward(C *S, const C *in, C *out, const MAP &m, const tw<T> *tb, int tid, bool scl, T sr,
+                               T si) {
+        load_vec(S, in, m, tid);
+        inner_stages<0>(S, tb, tid);
         __syncthreads();
-        if constexpr (s > 0) inverse_from<s - 1>(S, gm, p, tid);
+        edge_stage(S, out, m, tid, scl, sr, si);
+    }
+    // frequency side -> vector side
+    static ZM_DEV void inverse(C *S, const C *in, C *out, const MAP &m, const tw<T> *tb, int tid, bool scl, T sr,
+                               T si) {
+        edge_stage(S, const_cast<C *>(in), m, tid, false, T(1), T(0));
+        __syncthreads();
+        inner_stages<NST - 2>(S, tb, tid);
+        store_vec(S, out, m, tid, scl, sr, si);
     }
 };
 
@@ -221,19 +245,17 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
     using A = AxisPass<T, LN, LTL, LP, LE, INV>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T> *S = reinterpret_cast<cpx<T> *>(smem_raw);
-    const int tid = threadIdx.x;
     const LineAddr la = line_addr(p.g, p.kind, (int64_t)blockIdx.x << LTL, p.m.lg);
     const cpx<T> *in = reinterpret_cast<const cpx<T> *>(p.in);
     cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
-    const bool scl = p.apply_scale;
-    const T sr = (T)p.scale_re, si = (T)p.scale_im;
-    if constexpr (!INV) {
-        A::load_vec(S, in + la.a_base, p.m, tid);
-        A::template forward_from<0>(S, out + la.f_base, p, tid, scl, sr, si);
-    } else {
-        A::template inverse_from<A::NST - 1>(S, const_cast<cpx<T> *>(in) + la.f_base, p, tid);
-        A::store_vec(S, out + la.a_base, p.m, tid, scl, sr, si);
-    }
+    const tw<T> *tb = reinterpret_cast<const tw<T> *>(p.tw);
+    const AxisParamMap m{p.m};
+    if constexpr (!INV)
+        A::forward(S, in + la.a_base, out + la.f_base, m, tb, threadIdx.x, p.apply_scale, (T)p.scale_re,
+                   (T)p.scale_im);
+    else
+        A::inverse(S, in + la.f_base, out + la.a_base, m, tb, threadIdx.x, p.apply_scale, (T)p.scale_re,
+                   (T)p.scale_im);
 }
 
 template <typename T, int LN, int LTL, int LP, int LE, bool INV>
