@@ -364,6 +364,8 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     P->own_work = nullptr;
     P->twx = nullptr;
     P->axis[0][0].ltl = -1;
+    for (int r = 0; r < 2; r++)
+        for (int t = 0; t < 2; t++) P->perm[r][t] = zm::perm_map(g, dtype, r, t);
     std::vector<int64_t> exps;   // exponents of the axis pass' stage twiddles
     int ltl = 0, lp = 0, le = 0;
     if (!(flags & ZM_FLAG_PERMUTE_ONLY) && zm::axis_tile(g, dtype, total, &ltl, &lp, &le)) {

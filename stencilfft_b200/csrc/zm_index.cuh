@@ -1,4 +1,4 @@
-// zm_index.cuh -- device forms of the reference's index maps (zmodel/utils.h) on the
+// zm_index.cuh -- host and device forms of the reference's index maps (zmodel/utils.h) on the
 // interleaved layouts, and the counter-based field generators.
 #pragma once
 
@@ -8,20 +8,20 @@
 namespace zm {
 
 // lp / ct of utils.h:232-241 on powers of two
-ZM_DEV int64_t d_lp(int64_t i, const Geom &g) { return (i >> g.logVP) + ((i & (g.vp - 1)) << g.logM); }
-ZM_DEV int64_t d_ct(int64_t q, const Geom &g) { return ((q & (g.m - 1)) << g.logVEC) + (q >> g.logM); }
+ZM_HD int64_t d_lp(int64_t i, const Geom &g) { return (i >> g.logVP) + ((i & (g.vp - 1)) << g.logM); }
+ZM_HD int64_t d_ct(int64_t q, const Geom &g) { return ((q & (g.m - 1)) << g.logVEC) + (q >> g.logM); }
 
-ZM_DEV int64_t d_l2g(int64_t li, int64_t id, const Geom &g) {
+ZM_HD int64_t d_l2g(int64_t li, int64_t id, const Geom &g) {
     return ((li >> g.logB) << (g.logB + g.logP)) + (id << g.logB) + (li & (g.b - 1));
 }
-ZM_DEV int64_t d_pos2gc(int64_t pos, int64_t cid, const Geom &g) {
+ZM_HD int64_t d_pos2gc(int64_t pos, int64_t cid, const Geom &g) {
     const int64_t j = pos >> g.logVEC, jj = pos & (g.vec - 1);
     return (jj << (g.logB + g.logP)) + (cid << g.logB) + j;
 }
 
 struct Coords { int64_t r, l1, l2, pos, did, rid, cid; };
 
-ZM_DEV Coords coords(int64_t e, const Geom &g) {
+ZM_HD Coords coords(int64_t e, const Geom &g) {
     Coords c;
     const int64_t L = g.L;
     c.pos = e & (L - 1);
@@ -44,7 +44,7 @@ ZM_DEV Coords coords(int64_t e, const Geom &g) {
 }
 
 // global linear index held by interleaved element e of the real-space layout
-ZM_DEV int64_t real_gidx(int64_t e, const Geom &g) {
+ZM_HD int64_t real_gidx(int64_t e, const Geom &g) {
     Coords c = coords(e, g);
     const int64_t gc = d_pos2gc(c.pos, c.cid, g);
     const int64_t gr = d_l2g(c.l2, c.rid, g);
@@ -54,7 +54,7 @@ ZM_DEV int64_t real_gidx(int64_t e, const Geom &g) {
 }
 
 // frequency indices held by element e of the reciprocal layout
-ZM_DEV void recip_k(int64_t e, const Geom &g, int64_t &k0, int64_t &k1, int64_t &k2) {
+ZM_HD void recip_k(int64_t e, const Geom &g, int64_t &k0, int64_t &k1, int64_t &k2) {
     Coords c = coords(e, g);
     const int64_t L = g.L;
     if (g.dim == 2) {   // (ky, kx): kx from the local row, ky from the local column
@@ -67,7 +67,7 @@ ZM_DEV void recip_k(int64_t e, const Geom &g, int64_t &k0, int64_t &k1, int64_t 
         k0 = d_ct(c.did * L + d_lp(c.pos, g), g);
     }
 }
-ZM_DEV int64_t recip_gidx(int64_t e, const Geom &g) {
+ZM_HD int64_t recip_gidx(int64_t e, const Geom &g) {
     int64_t k0, k1, k2;
     recip_k(e, g, k0, k1, k2);
     return g.dim == 2 ? (k1 << g.logN) + k2 : (((k0 << g.logN) + k1) << g.logN) + k2;

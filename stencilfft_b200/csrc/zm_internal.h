@@ -67,6 +67,7 @@ cudaError_t launch_stencil(const zm_plan_s *p, int op, bool real_field, const vo
                            double coef2 = 1.0);
 
 // zm_layout.cu
+PermMap perm_map(const Geom &g, int dtype, bool reciprocal, bool to_natural);
 cudaError_t launch_convert(const zm_plan_s *p, bool reciprocal, bool to_natural, const void *in,
                            void *out, cudaStream_t st);
 cudaError_t launch_spectral(const zm_plan_s *p, void *data, int op, double a, cudaStream_t st);

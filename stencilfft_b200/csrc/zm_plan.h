@@ -74,6 +74,20 @@ struct AxisParams {
     AxisMap m;
 };
 
+// A layout conversion as a bit permutation (zm_layout.cu): tiles of 2^le elements.
+struct PermMap {
+    int le;
+    // tile bits in the order of the input's (ia, is) and the output's (oa, os) addresses:
+    // address bit, shared-memory slot
+    unsigned char ia[12], oa[12];
+    short is[12], os[12];
+    // block index: fields of its bits (mask) that move to fin bits up (input) and, shifted
+    // down by flow, to bit fout (output)
+    int nf;
+    unsigned fmask[24];
+    unsigned char fin[24], flow[24], fout[24];
+};
+
 }  // namespace zm
 
 struct zm_plan_s {
@@ -96,5 +110,6 @@ struct zm_plan_s {
     // a workspace (its own row interleave)
     zm::AxisMap axis[2][3];
     void *twx;        // its stage twiddles (inside the tables allocation)
+    zm::PermMap perm[2][2];   // converters [reciprocal][to natural]
     void *own_work;   // ZM_FLAG_OWN_WORKSPACE: one field, used by transforms called with work = NULL
 };
