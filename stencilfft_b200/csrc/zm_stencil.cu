@@ -252,11 +252,13 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
     const int64_t vi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (vi >= nthreads) return;
     const int L = (int)g.L, N = (int)g.n, P = (int)g.p;
-    const int vrow_n = L / K;                    // vectors per row
-    const int vpos = (int)(vi % vrow_n);
-    const int64_t rest = vi / vrow_n;
-    const int rg = (int)(rest % (L / RY));
-    const int rank = (int)(rest / (L / RY));
+    // powers of two: shifts (64-bit divisions here were half the FP64 kernels' instructions)
+    constexpr int logK = K == 4 ? 2 : K == 2 ? 1 : 0, logRY = RY == 4 ? 2 : RY == 2 ? 1 : 0;
+    const int logV = g.logL - logK, logG = g.logL - logRY;   // vectors per row, row groups per rank
+    const int vpos = (int)vi & ((1 << logV) - 1);
+    const int64_t rest = vi >> logV;
+    const int rg = (int)rest & ((1 << logG) - 1);
+    const int rank = (int)(rest >> logG);
     const int lr0 = rg * RY, pos = vpos * K;
     const int64_t e0 = ((int64_t)rank << (2 * g.logL)) + (int64_t)lr0 * L + pos;
     const int cid = rank & (P - 1), rid = rank >> g.logP;
