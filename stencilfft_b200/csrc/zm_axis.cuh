@@ -57,6 +57,41 @@ template <typename T, int LN, int LTL, int LP, int LE> struct AxisCfg {
     static constexpr int BY_SMEM = (int)((size_t)227 * 1024 / (SMEM + 1024));
     static constexpr int MINB0 = BY_REG < BY_SMEM ? BY_REG : BY_SMEM;
     static constexpr int MINB = MINB0 < 1 ? 1 : (MINB0 > 16 ? 16 : MINB0);
+
+    // Twiddles kept in tensor memory by the persistent form: a thread's entries of stage s are
+    // the rows k = 1 .. R - 1 of its HI index values, four words each, in its own lane.
+    static constexpr int units(int s) {
+        const int lu = LP - axis_lr(LN, LE, s);
+        return 1 << (lu - (LTL < lu ? LTL : lu));
+    }
+    static constexpr int words(int s) { return 4 * ((1 << axis_lr(LN, LE, s)) - 1) * units(s); }
+    // 512 columns hold NT / 128 threads per lane and MINB CTAs per SM
+    static constexpr int BUDGET = NT >= 128 ? 512 / MINB / (NT / 128) : 0;
+    // stages in tensor memory: from the last one back, as many as fit
+    static constexpr int first_tm() {
+        int w = 0, s = NST - 1;
+        while (s > 0 && w + (words(s - 1) + 15) / 16 * 16 <= BUDGET) w += (words(--s) + 15) / 16 * 16;
+        return s;
+    }
+    static constexpr int TM0 = first_tm();
+    static constexpr int tm_at(int s) {   // first column of stage s in a thread's share
+        int w = 0;
+        for (int q = TM0; q < s; q++) w += (words(q) + 15) / 16 * 16;
+        return w;
+    }
+    static constexpr int SHARE = tm_at(NST - 1);
+    static constexpr int cols() {
+        int c = 32;
+        while (c < SHARE * (NT / 128)) c *= 2;
+        return c;
+    }
+    // The persistent form is for tiles that leave room for one CTA per SM, where nothing else
+    // covers a tile's loads: N = 8192 c64 701 / 728 -> 664 / 669 us forward / inverse, c128
+    // 1402 / 1535 -> 1198 / 1393 (twiddles in tensor memory alone 695 / 730 and 1354 / 1479).
+    // With two CTAs or more it is no faster (N = 4096 c64 136 / 160 against 142 / 159, 3D
+    // N = 256 c64 156 / 159 against 175 / 177), nor on one-line complex64 tiles of 2^14
+    // points, whose strided side moves single elements (4266 / 3520 against 4472 / 4342).
+    static constexpr bool TM_OK = MINB == 1 && LN == 13 && TM0 < NST - 1 && cols() <= 512;
 };
 
 // The weight tables as the kernel sees them: launch parameters, or a table in global memory
@@ -104,7 +139,8 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
 
     // global vector side <-> tile, in address order: thread bits first; complex64 keeps the
     // lowest address bit in the registers (16-byte accesses)
-    static ZM_DEV void load_vec(C *S, const C *in, const MAP &m, int tid) {
+    // BAR: a barrier between the loads and the tile's first write (the tile is still being read)
+    template <bool BAR = false> static ZM_DEV void load_vec(C *S, const C *in, const MAP &m, int tid) {
         in += axis_bits<LNT>(tid, [&](int b) { return m.va(b); });
         S += axis_bits<LNT>(tid, [&](int b) { return m.vs(b); });
         auto ra = [&](int r) { return axis_bits<LP>(r, [&](int b) { return m.va(LNT + b); }); };
@@ -122,8 +158,28 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
 #pragma unroll
             for (int r = 0; r < EPT; r++) v[r] = MAP::CONST_IN ? ldg(in + ra(r)) : in[ra(r)];
         }
+        if constexpr (BAR) __syncthreads();
 #pragma unroll
         for (int r = 0; r < EPT; r++) S[rs(r)] = v[r];
+    }
+    // this thread's share of the next tile into L2
+    static ZM_DEV void prefetch(const void *p) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((unsigned long long)__cvta_generic_to_global(p)));
+    }
+    static ZM_DEV void prefetch_vec(const C *in, const MAP &m, int tid) {
+        in += axis_bits<LNT>(tid, [&](int b) { return m.va(b); });
+#pragma unroll
+        for (int r = 0; r < EPT; r += sizeof(T) == 4 ? 2 : 1)
+            prefetch(in + axis_bits<LP>(r, [&](int b) { return m.va(LNT + b); }));
+    }
+    static ZM_DEV void prefetch_edge(const C *gm, const MAP &m, int tid) {
+        constexpr int lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, LU = LP - lr;
+        gm += axis_bits<LNT>(tid, [&](int b) { return m.fa(b); });
+#pragma unroll
+        for (int u = 0; u < 1 << LU; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                prefetch(gm + axis_bits<LU>(u, [&](int b) { return m.fa(LNT + b); }) + axis_bits<lr>(r, [&](int b) { return m.fr(b); }));
     }
     static ZM_DEV void store_vec(const C *S, C *out, const MAP &m, int tid, bool scl, T sr, T si) {
         out += axis_bits<LNT>(tid, [&](int b) { return m.va(b); });
@@ -147,7 +203,7 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
 
     // The stage next to the frequency side (the last one forward, the first inverse): units
     // in frequency-side order, global memory at `gm` on that side.
-    static ZM_DEV void edge_stage(C *S, C *gm, const MAP &m, int tid, bool scl, T sr, T si) {
+    template <bool BAR = false> static ZM_DEV void edge_stage(C *S, C *gm, const MAP &m, int tid, bool scl, T sr, T si) {
         constexpr int lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, LU = LP - lr;
         gm += axis_bits<LNT>(tid, [&](int b) { return m.fa(b); });
         S += axis_bits<LNT>(tid, [&](int b) { return m.fs(b); });
@@ -163,6 +219,8 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
                 else x[r] = s[axis_slot(r << LTL)];
             }
             dft<R, DIR, T, COMP>(x);
+            if constexpr (BAR && INV)
+                if (u == 0) __syncthreads();
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 if constexpr (INV) {
@@ -175,18 +233,24 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
         }
     }
     // An inner stage: thread -> (low line bits, v, index bits above the digit); the units of
-    // one `h` differ in the highest line bits only and share their twiddles.
-    template <int s> static ZM_DEV void inner_stage(C *S, const tw<T> *tb, int tid) {
-        constexpr int lr = axis_lr(LN, LE, s), sh = axis_sh(LN, LE, s), shp = sh + LTL, R = 1 << lr, LU = LP - lr;
-        constexpr int LUT = LTL < LU ? LTL : LU, LT0 = LTL - LUT, HI = 1 << (LU - LUT), LO = 1 << LUT;
+    // one `h` differ in the highest line bits only and share their twiddles.  TM: the
+    // twiddles come from the thread's share of tensor memory at `tm`, else from the table.
+    template <int s> struct Inner {
+        static constexpr int lr = axis_lr(LN, LE, s), sh = axis_sh(LN, LE, s), shp = sh + LTL, R = 1 << lr, LU = LP - lr;
+        static constexpr int LUT = LTL < LU ? LTL : LU, LT0 = LTL - LUT, HI = 1 << (LU - LUT), LO = 1 << LUT;
+        static ZM_DEV int iv(int tid, int h) { return (tid + h * NT) >> LT0; }   // (bits above the digit, v)
+        static ZM_DEV int v(int tid, int h) { return iv(tid, h) & ((1 << sh) - 1); }
+    };
+    template <int s, bool TM> static ZM_DEV void inner_stage(C *S, const tw<T> *tb, uint32_t tm, int tid) {
+        using G = Inner<s>;
+        constexpr int R = G::R, HI = G::HI, LO = G::LO, LT0 = G::LT0, sh = G::sh, shp = G::shp, lr = G::lr;
+        constexpr bool MEM = TM && s >= CF::TM0;
         tb += axis_tw(LN, LE, s);
 #pragma unroll
         for (int h = 0; h < HI; h++) {
-            const int U = tid + h * NT;
-            const int iv = U >> LT0;                       // (bits above the digit, v)
-            const int v = iv & ((1 << sh) - 1);
+            const int iv = G::iv(tid, h), v = G::v(tid, h);
             const int i = ((iv >> sh) << (sh + lr)) | v;
-            const int slot = axis_slot((i << LTL) | (U & ((1 << LT0) - 1)));
+            const int slot = axis_slot((i << LTL) | ((tid + h * NT) & ((1 << LT0) - 1)));
             C x[LO][R];
 #pragma unroll
             for (int q = 0; q < LO; q++) {
@@ -194,11 +258,29 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
                 for (int r = 0; r < R; r++) x[q][r] = S[slot + axis_slot(q << LT0 | r << shp)];
             }
             auto twiddle = [&]() {
+                if constexpr (MEM) {
+                    // entry h (R - 1) + r - 1 of the stage, four entries per 16 columns
 #pragma unroll
-                for (int r = 1; r < R; r++) {
-                    const tw<T> w = ldtw(tb, (r << sh) + v);
+                    for (int c = h * (R - 1) / 4; c <= ((h + 1) * (R - 1) - 1) / 4; c++) {
+                        uint32_t w16[16];
+                        tmem_ld16(tm + CF::tm_at(s) + 16 * c, w16);
 #pragma unroll
-                    for (int q = 0; q < LO; q++) x[q][r] = twmul<INV>(x[q][r], w);
+                        for (int e = 0; e < 4; e++) {
+                            const int r = 4 * c + e - h * (R - 1) + 1;
+                            if (r < 1 || r >= R) continue;
+                            tw<T> w;
+                            memcpy(&w, w16 + 4 * e, 16);
+#pragma unroll
+                            for (int q = 0; q < LO; q++) x[q][r] = twmul<INV>(x[q][r], w);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 1; r < R; r++) {
+                        const tw<T> w = ldtw(tb, (r << sh) + v);
+#pragma unroll
+                        for (int q = 0; q < LO; q++) x[q][r] = twmul<INV>(x[q][r], w);
+                    }
                 }
             };
             if constexpr (INV) twiddle();
@@ -212,30 +294,56 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
             }
         }
     }
-    // stages s .. NST - 2 forward, s .. 0 inverse, a barrier before / after each
-    template <int s> static ZM_DEV void inner_stages(C *S, const tw<T> *tb, int tid) {
-        if constexpr (s >= 0 && s < NST - 1) {
-            if constexpr (!INV) __syncthreads();
-            inner_stage<s>(S, tb, tid);
-            if constexpr (INV) __syncthreads();
-            inner_stages<(INV ? s - 1 : s + 1)>(S, tb, tid);
+    // this thread's entries of stages s .. into its share of tensor memory
+    template <int s> static ZM_DEV void park_twiddles(const tw<T> *tb, uint32_t tm, int tid) {
+        if constexpr (s < NST - 1) {
+            using G = Inner<s>;
+            constexpr int NE = (G::R - 1) * G::HI;
+            const tw<T> *t = tb + axis_tw(LN, LE, s);
+#pragma unroll 1
+            for (int c = 0; c < (NE + 3) / 4; c++) {
+                uint32_t w16[16];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int n = 4 * c + e < NE ? 4 * c + e : NE - 1;
+                    const int h = n / (G::R - 1), r = n % (G::R - 1) + 1;
+                    const tw<T> w = ldtw(t, (r << G::sh) + G::v(tid, h));
+                    memcpy(w16 + 4 * e, &w, 16);
+                }
+                tmem_st16(tm + CF::tm_at(s) + 16 * c, w16);
+            }
+            park_twiddles<s + 1>(tb, tm, tid);
         }
     }
-    // vector side -> frequency side
-    static ZM_DEV void forward(C *S, const C *in, C *out, const MAP &m, const tw<T> *tb, int tid, bool scl, T sr,
-                               T si) {
-        load_vec(S, in, m, tid);
-        inner_stages<0>(S, tb, tid);
-        __syncthreads();
-        edge_stage(S, out, m, tid, scl, sr, si);
+    // stages s .. NST - 2 forward, s .. 0 inverse, a barrier before / after each
+    template <int s, bool TM = false> static ZM_DEV void inner_stages(C *S, const tw<T> *tb, int tid, uint32_t tm = 0) {
+        if constexpr (s >= 0 && s < NST - 1) {
+            if constexpr (!INV) __syncthreads();
+            inner_stage<s, TM>(S, tb, tm, tid);
+            if constexpr (INV) __syncthreads();
+            inner_stages<(INV ? s - 1 : s + 1), TM>(S, tb, tid, tm);
+        }
     }
-    // frequency side -> vector side
-    static ZM_DEV void inverse(C *S, const C *in, C *out, const MAP &m, const tw<T> *tb, int tid, bool scl, T sr,
-                               T si) {
-        edge_stage(S, const_cast<C *>(in), m, tid, false, T(1), T(0));
-        __syncthreads();
-        inner_stages<NST - 2>(S, tb, tid);
-        store_vec(S, out, m, tid, scl, sr, si);
+    // one tile, vector side -> frequency side (forward) or back; TM: persistent form, the
+    // previous tile may still be read when this one starts
+    template <bool TM = false>
+    static ZM_DEV void run(C *S, const C *in, C *out, const MAP &m, const tw<T> *tb, int tid, bool scl, T sr, T si,
+                           uint32_t tm = 0, const C *next = nullptr) {
+        if constexpr (!INV) {
+            load_vec<TM>(S, in, m, tid);
+            if constexpr (TM)
+                if (next) prefetch_vec(next, m, tid);
+            inner_stages<0, TM>(S, tb, tid, tm);
+            __syncthreads();
+            edge_stage(S, out, m, tid, scl, sr, si);
+        } else {
+            edge_stage<TM>(S, const_cast<C *>(in), m, tid, false, T(1), T(0));
+            if constexpr (TM)
+                if (next) prefetch_edge(next, m, tid);
+            __syncthreads();
+            inner_stages<NST - 2, TM>(S, tb, tid, tm);
+            store_vec(S, out, m, tid, scl, sr, si);
+        }
     }
 };
 
@@ -250,12 +358,47 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
     cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
     const tw<T> *tb = reinterpret_cast<const tw<T> *>(p.tw);
     const AxisParamMap m{p.m};
-    if constexpr (!INV)
-        A::forward(S, in + la.a_base, out + la.f_base, m, tb, threadIdx.x, p.apply_scale, (T)p.scale_re,
-                   (T)p.scale_im);
-    else
-        A::inverse(S, in + la.f_base, out + la.a_base, m, tb, threadIdx.x, p.apply_scale, (T)p.scale_re,
-                   (T)p.scale_im);
+    A::run(S, in + (INV ? la.f_base : la.a_base), out + (INV ? la.a_base : la.f_base), m, tb, threadIdx.x,
+           p.apply_scale, (T)p.scale_re, (T)p.scale_im);
+}
+
+// The persistent form, one CTA per SM: CTA c walks tiles c, c + CTAs, ..., each thread's stage
+// twiddles (the same for every tile) in tensor memory, and asks for its next tile in L2 as
+// soon as it holds the current one.
+template <typename T, int LN, int LTL, int LP, int LE, bool INV>
+__global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T, LN, LTL, LP, LE>::MINB))
+    axis_tm_kernel(const __grid_constant__ AxisParams p, unsigned tiles) {
+    using A = AxisPass<T, LN, LTL, LP, LE, INV>;
+    using CF = typename A::CF;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint32_t s_tm;
+    cpx<T> *S = reinterpret_cast<cpx<T> *>(smem_raw);
+    const int tid = threadIdx.x;
+    const tw<T> *tb = reinterpret_cast<const tw<T> *>(p.tw);
+    if (tid < 32) tmem_alloc(&s_tm, CF::cols());
+    __syncthreads();
+    tmem_fence_after();
+    const uint32_t tm0 = s_tm;
+    // warp w reaches lanes 32 (w mod 4) ..; its column share is number w / 4
+    const uint32_t tm = tm0 + ((uint32_t)(tid >> 5 & 3) << 21) + (uint32_t)(tid >> 7) * CF::SHARE;
+    A::template park_twiddles<CF::TM0>(tb, tm, tid);
+    const cpx<T> *in = reinterpret_cast<const cpx<T> *>(p.in);
+    cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
+    const AxisParamMap m{p.m};
+#pragma unroll 1
+    for (unsigned c = blockIdx.x; c < tiles; c += gridDim.x) {
+        const LineAddr la = line_addr(p.g, p.kind, (int64_t)c << LTL, p.m.lg);
+        const cpx<T> *nx = nullptr;
+        if (c + gridDim.x < tiles) {
+            const LineAddr ln = line_addr(p.g, p.kind, (int64_t)(c + gridDim.x) << LTL, p.m.lg);
+            nx = in + (INV ? ln.f_base : ln.a_base);
+        }
+        A::template run<true>(S, in + (INV ? la.f_base : la.a_base), out + (INV ? la.a_base : la.f_base), m, tb, tid,
+                              p.apply_scale, (T)p.scale_re, (T)p.scale_im, tm, nx);
+    }
+    tmem_fence_before();
+    __syncthreads();
+    if (tid < 32) tmem_dealloc(tm0, CF::cols());
 }
 
 template <typename T, int LN, int LTL, int LP, int LE, bool INV>
@@ -272,7 +415,28 @@ cudaError_t launch_axis(const AxisParams &p, int64_t nlines, cudaStream_t st) {
             if (dev < 64) done[dev] = true;
         }
     }
-    kern<<<(unsigned)(nlines >> LTL), CF::NT, CF::SMEM, st>>>(p);
+    const unsigned tiles = (unsigned)(nlines >> LTL);
+    if constexpr (CF::TM_OK) {
+        static int resident[64] = {0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        auto ktm = axis_tm_kernel<T, LN, LTL, LP, LE, INV>;
+        int ctas = dev < 64 ? resident[dev] : 0;
+        if (!ctas) {
+            int sms = 0;
+            cudaError_t e = cudaFuncSetAttribute(ktm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return e;
+            ctas = sms;   // one per SM
+            if (dev < 64) resident[dev] = ctas;
+        }
+        if (tiles >= 3 * (unsigned)ctas) {
+            ktm<<<(unsigned)ctas, CF::NT, CF::SMEM, st>>>(p, tiles);
+            count_launch();
+            return cudaGetLastError();
+        }
+    }
+    kern<<<tiles, CF::NT, CF::SMEM, st>>>(p);
     count_launch();
     return cudaGetLastError();
 }

@@ -78,9 +78,9 @@ __device__ __noinline__ void batch_axis_tile(int op, cpx<T> *S, const cpx<T> *in
     const int tid = threadIdx.x;
     const LineAddr la = line_addr(g, xpass ? PASS_X2 : PASS_Y2, l0, __ldg(&map->lg));
     if (op == ATILE_FWD) {
-        AF::forward(S, in + la.a_base, out + la.f_base, m, tb, tid, false, T(1), T(0));
+        AF::run(S, in + la.a_base, out + la.f_base, m, tb, tid, false, T(1), T(0));
     } else if (op == ATILE_INV) {
-        AI::inverse(S, in + la.f_base, out + la.a_base, m, tb, tid, scale != T(1), scale, T(0));
+        AI::run(S, in + la.f_base, out + la.a_base, m, tb, tid, scale != T(1), scale, T(0));
     } else {
         AF::load_vec(S, in + la.a_base, m, tid);
         AF::template inner_stages<0>(S, tb, tid);
