@@ -447,10 +447,12 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
     }
 }
 
-// The kernels: the default register allocation (four rows per thread, FP32), and one
-// row per thread in FP64 held to 51 registers, five CTAs per SM (the FP64 kernel waits on
-// its loads: 56 registers and four CTAs per SM left the three stencils at 4.01 ms at
-// N = 16384 c128, five take 3.72 ms)
+// The kernels: the default register allocation (four rows per thread, FP32), and a stated
+// minimum of CTAs per SM, five where a thread holds one or two rows in FP64 (51 registers:
+// the kernel waits on its loads; four CTAs left the three stencils at 4.01 ms at N = 16384
+// c128 against 3.72).  Multiplying by a precomputed reciprocal and correcting the remainder
+// in place of the FP64 division was slower (dx 113 -> 121 us at N = 4096: the division's own
+// fast path is as short as the range checks that this takes).
 template <typename S, int NC, int OP, int RY>
 __global__ void __launch_bounds__(256) stencil_rows_kernel(const S *__restrict__ in, S *__restrict__ out,
                                                            S *__restrict__ out2, S *__restrict__ out3,
@@ -458,12 +460,12 @@ __global__ void __launch_bounds__(256) stencil_rows_kernel(const S *__restrict__
                                                            S rden) {
     stencil_rows_body<S, NC, OP, RY>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
 }
-template <typename S, int NC, int OP>
-__global__ void __launch_bounds__(256, 5) stencil_rows1_kernel(const S *__restrict__ in, S *__restrict__ out,
+template <typename S, int NC, int OP, int RY, int MB>
+__global__ void __launch_bounds__(256, MB) stencil_rowsb_kernel(const S *__restrict__ in, S *__restrict__ out,
                                                                S *__restrict__ out2, S *__restrict__ out3,
                                                                const Geom g, int64_t nthreads, S coef, S coef2,
                                                                S rden) {
-    stencil_rows_body<S, NC, OP, 1>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
+    stencil_rows_body<S, NC, OP, RY>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
 }
 
 // 3D Laplacian (laplace3d.cu:98-224 accumulation order) with RX vectors of one line per
@@ -910,31 +912,36 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
     const double dl = op == ST_ALL ? coef2 : coef;
     const S rd = (S)(1.0 / (12.0 * dl));
     if (p->g.dim == 2) {
-        if (sizeof(S) == 4 && p->g.b % 4 == 0) {
-            // four rows of a B-row block per thread (FP32)
-            const int64_t nt = nvec / 4;
-            const unsigned g4 = (unsigned)((nt + threads - 1) / threads);
-            if (op == ST_LAPLACE)
-                stencil_rows_kernel<S, NC, ST_LAPLACE, 4><<<g4, threads, 0, st>>>(i, o, o2, o3, p->g, nt, c, c2, rd);
-            else if (op == ST_DX)
-                stencil_rows_kernel<S, NC, ST_DX, 4><<<g4, threads, 0, st>>>(i, o, o2, o3, p->g, nt, c, c2, rd);
-            else if (op == ST_DY)
-                stencil_rows_kernel<S, NC, ST_DY, 4><<<g4, threads, 0, st>>>(i, o, o2, o3, p->g, nt, c, c2, rd);
-            else
-                stencil_rows_kernel<S, NC, ST_ALL, 4><<<g4, threads, 0, st>>>(i, o, o2, o3, p->g, nt, c, c2, rd);
-        } else if (sizeof(S) == 8) {
-            // FP64: one row per thread, rows of the same B-row block addressed directly, five
-            // CTAs per SM (two rows per thread, 70 registers, were slower: 4.20 -> 4.54 ms at
-            // N = 16384 for the three stencils in one launch; four rows 4.34 ms)
-            const unsigned g1 = (unsigned)((nvec + threads - 1) / threads);
-            if (op == ST_LAPLACE)
-                stencil_rows1_kernel<S, NC, ST_LAPLACE><<<g1, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
-            else if (op == ST_DX)
-                stencil_rows1_kernel<S, NC, ST_DX><<<g1, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
-            else if (op == ST_DY)
-                stencil_rows1_kernel<S, NC, ST_DY><<<g1, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
-            else
-                stencil_rows1_kernel<S, NC, ST_ALL><<<g1, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+        auto blocks = [&](int ry) { return (unsigned)((nvec / ry + threads - 1) / threads); };
+#define ZM_ROWS(OP, RY) \
+    stencil_rows_kernel<S, NC, OP, RY><<<blocks(RY), threads, 0, st>>>(i, o, o2, o3, p->g, nvec / RY, c, c2, rd)
+#define ZM_ROWSB(OP, RY, MB) \
+    stencil_rowsb_kernel<S, NC, OP, RY, MB><<<blocks(RY), threads, 0, st>>>(i, o, o2, o3, p->g, nvec / RY, c, c2, rd)
+        if constexpr (sizeof(S) == 8) {
+            // FP64, us at N = 4096, P = 4, B = 64, c128 / real field.  dy, whose outputs share
+            // rows: four rows of a B-row block per thread (118 / 60 with one row, 96 / 52 with
+            // two, 86 / 45 with four).  Laplacian: two rows (109 -> 104; at B = 4, 129 -> 131,
+            // one row stays better).  dx shares no rows (113 with one, 119 with two), and the
+            // three in one launch hold too many registers with more than one (221 against 238).
+            if (op == ST_DY && p->g.b % 4 == 0) ZM_ROWSB(ST_DY, 4, 4);
+            else if (op == ST_DY && p->g.b % 2 == 0) ZM_ROWSB(ST_DY, 2, 5);
+            else if (op == ST_DY) ZM_ROWSB(ST_DY, 1, 5);
+            else if (op == ST_LAPLACE && p->g.b % 8 == 0) ZM_ROWSB(ST_LAPLACE, 2, 5);
+            else if (op == ST_LAPLACE) ZM_ROWSB(ST_LAPLACE, 1, 5);
+            else if (op == ST_DX) ZM_ROWSB(ST_DX, 1, 5);
+            else ZM_ROWSB(ST_ALL, 1, 5);
+        } else if (p->g.b % 4 == 0) {
+            // FP32: four rows of a B-row block per thread
+            if (op == ST_LAPLACE) ZM_ROWS(ST_LAPLACE, 4);
+            else if (op == ST_DX) ZM_ROWS(ST_DX, 4);
+            else if (op == ST_DY) ZM_ROWS(ST_DY, 4);
+            else ZM_ROWS(ST_ALL, 4);
+        } else if (p->g.b == 2 && op == ST_DX) {
+            // FP32 at B = 2, N = 4096, P = 2: two rows per thread, dx 98 -> 88 us, the three in
+            // one launch 155 -> 136; the Laplacian is slower that way (80 -> 92)
+            ZM_ROWSB(ST_DX, 2, 4);
+        } else if (p->g.b == 2 && op == ST_ALL) {
+            ZM_ROWSB(ST_ALL, 2, 4);
         } else if (op == ST_LAPLACE)
             stencil_kernel<S, NC, ST_LAPLACE, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
         else if (op == ST_DX)
@@ -943,6 +950,8 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
             stencil_kernel<S, NC, ST_DY, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
         else
             stencil_kernel<S, NC, ST_ALL, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+#undef ZM_ROWS
+#undef ZM_ROWSB
     } else {
         if (op != ST_LAPLACE) return cudaErrorInvalidValue;
         if (NC == 2) {
