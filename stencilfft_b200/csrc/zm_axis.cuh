@@ -353,11 +353,13 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
     using A = AxisPass<T, LN, LTL, LP, LE, INV>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T> *S = reinterpret_cast<cpx<T> *>(smem_raw);
+    overlap_next();
     const LineAddr la = line_addr(p.g, p.kind, (int64_t)blockIdx.x << LTL, p.m.lg);
     const cpx<T> *in = reinterpret_cast<const cpx<T> *>(p.in);
     cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
     const tw<T> *tb = reinterpret_cast<const tw<T> *>(p.tw);
     const AxisParamMap m{p.m};
+    overlap_wait();
     A::run(S, in + (INV ? la.f_base : la.a_base), out + (INV ? la.a_base : la.f_base), m, tb, threadIdx.x,
            p.apply_scale, (T)p.scale_re, (T)p.scale_im);
 }
@@ -382,6 +384,8 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
     // warp w reaches lanes 32 (w mod 4) ..; its column share is number w / 4
     const uint32_t tm = tm0 + ((uint32_t)(tid >> 5 & 3) << 21) + (uint32_t)(tid >> 7) * CF::SHARE;
     A::template park_twiddles<CF::TM0>(tb, tm, tid);
+    overlap_next();
+    overlap_wait();
     const cpx<T> *in = reinterpret_cast<const cpx<T> *>(p.in);
     cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
     const AxisParamMap m{p.m};
@@ -431,14 +435,12 @@ cudaError_t launch_axis(const AxisParams &p, int64_t nlines, cudaStream_t st) {
             if (dev < 64) resident[dev] = ctas;
         }
         if (tiles >= 3 * (unsigned)ctas) {
-            ktm<<<(unsigned)ctas, CF::NT, CF::SMEM, st>>>(p, tiles);
             count_launch();
-            return cudaGetLastError();
+            return launch_overlapped(ktm, (unsigned)ctas, CF::NT, CF::SMEM, st, p, tiles);
         }
     }
-    kern<<<tiles, CF::NT, CF::SMEM, st>>>(p);
     count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(kern, tiles, CF::NT, CF::SMEM, st, p);
 }
 
 }  // namespace zm

@@ -125,6 +125,16 @@ ZM_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memor
 ZM_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 ZM_DEV void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }   // all but the newest group
 
+// ------------------------------------------------ overlapped launches (launch_overlapped)
+// Let the next kernel of the stream be scheduled as this one's CTAs leave; wait until every
+// earlier kernel has finished and its writes are visible.  Every thread waits before its
+// first access to a field, so a kernel only ever overlaps another's scheduling and index
+// arithmetic.  Only the axis passes let the next kernel in early: from the 3D Laplacian, whose
+// CTAs walk long columns, its waiting CTAs took resources (3D N = 512 c64 round trip +
+// Laplacian 3.00 -> 3.58 ms); the other kernels only wait.
+ZM_DEV void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+ZM_DEV void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------ tensor memory (TMEM) staging
 // 128 lanes x 512 columns of 32 bits per SM.  With the 32x32b shape, warp w reaches the
 // 32 lanes 32 (w % 4) .. 32 (w % 4) + 31, lane i of the warp its own lane; an address is

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(256) permute_kernel(const cpx<T> *__restrict__
         return o;
     };
     cpx<T> v[EPT];
+    overlap_wait();
 #pragma unroll
     for (int r = 0; r < EPT; r += 1 + R0) {
         if constexpr (PAIR) {
@@ -173,9 +174,10 @@ PermMap perm_map(const Geom &g, int dtype, bool reciprocal, bool to_natural) {
 }
 
 template <typename T, int LE>
-static void launch_permute(const PermMap &m, int64_t tiles, const void *in, void *out, cudaStream_t st) {
-    permute_kernel<T, LE><<<(unsigned)tiles, LE < 8 ? 1 << LE : 256, 0, st>>>(
-        reinterpret_cast<const cpx<T> *>(in), reinterpret_cast<cpx<T> *>(out), m);
+static cudaError_t launch_permute(const PermMap &m, int64_t tiles, const void *in, void *out, cudaStream_t st) {
+    count_launch();
+    return launch_overlapped(permute_kernel<T, LE>, (unsigned)tiles, LE < 8 ? 1 << LE : 256, 0, st,
+                             reinterpret_cast<const cpx<T> *>(in), reinterpret_cast<cpx<T> *>(out), m);
 }
 
 cudaError_t launch_convert(const zm_plan_s *p, bool reciprocal, bool to_natural, const void *in,
@@ -183,7 +185,7 @@ cudaError_t launch_convert(const zm_plan_s *p, bool reciprocal, bool to_natural,
     const PermMap &m = p->perm[reciprocal][to_natural];
     const int64_t tiles = p->total >> m.le;
 #define ZM_PERM(T, LE) \
-    case LE: launch_permute<T, LE>(m, tiles, in, out, st); break;
+    case LE: return launch_permute<T, LE>(m, tiles, in, out, st);
     if (p->dtype == 0) {
         switch (m.le) {
             ZM_PERM(double, 2) ZM_PERM(double, 4) ZM_PERM(double, 6) ZM_PERM(double, 8) ZM_PERM(double, 9)
@@ -198,8 +200,6 @@ cudaError_t launch_convert(const zm_plan_s *p, bool reciprocal, bool to_natural,
         }
     }
 #undef ZM_PERM
-    count_launch();
-    return cudaGetLastError();
 }
 
 // --------------------------------------------------------- spectral operators
@@ -231,6 +231,7 @@ template <typename T, typename I>
 __global__ void __launch_bounds__(256) spectral_kernel(cpx<T> *__restrict__ d, const Geom g, int64_t total, int op,
                                                        double a) {
     const int64_t e0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * CEPT;
+    overlap_wait();
     if (e0 >= total) return;
     cpx<T> v[CEPT];
     ld_run(d + e0, v);
@@ -265,19 +266,17 @@ __global__ void __launch_bounds__(256) spectral_kernel(cpx<T> *__restrict__ d, c
 }
 
 template <typename T>
-static void spectral_t(const zm_plan_s *p, void *data, int op, double a, cudaStream_t st) {
+static cudaError_t spectral_t(const zm_plan_s *p, void *data, int op, double a, cudaStream_t st) {
     const int threads = 256;
     const unsigned grid = (unsigned)((p->total / CEPT + threads - 1) / threads);
     cpx<T> *d = reinterpret_cast<cpx<T> *>(data);
-    if (p->g.logN <= 14) spectral_kernel<T, int32_t><<<grid, threads, 0, st>>>(d, p->g, p->total, op, a);
-    else spectral_kernel<T, int64_t><<<grid, threads, 0, st>>>(d, p->g, p->total, op, a);
+    count_launch();
+    return launch_overlapped(p->g.logN <= 14 ? spectral_kernel<T, int32_t> : spectral_kernel<T, int64_t>, grid,
+                             threads, 0, st, d, p->g, p->total, op, a);
 }
 
 cudaError_t launch_spectral(const zm_plan_s *p, void *data, int op, double a, cudaStream_t st) {
-    if (p->dtype == 0) spectral_t<double>(p, data, op, a, st);
-    else spectral_t<float>(p, data, op, a, st);
-    count_launch();
-    return cudaGetLastError();
+    return p->dtype == 0 ? spectral_t<double>(p, data, op, a, st) : spectral_t<float>(p, data, op, a, st);
 }
 
 template <typename T>

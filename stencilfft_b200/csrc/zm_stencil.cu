@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
     using V = vec16<S>;
     constexpr int K = V::n / NC;                 // elements per vector
     const int64_t vi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    overlap_wait();
     if (vi >= nvec) return;
     const int64_t e = vi * K;                    // first element
     const int L = (int)g.L;
@@ -250,6 +251,7 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
     using V = vec16<S>;
     constexpr int K = V::n / NC;                 // elements per vector
     const int64_t vi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    overlap_wait();
     if (vi >= nthreads) return;
     const int L = (int)g.L, N = (int)g.n, P = (int)g.p;
     // powers of two: shifts (64-bit divisions here were half the FP64 kernels' instructions)
@@ -479,6 +481,7 @@ __global__ void __launch_bounds__(256, MB) stencil_rowsb_kernel(const S *__restr
 template <typename S, int NC, int RX>
 __global__ void __launch_bounds__(256) stencil3d_lines_kernel(const S *__restrict__ in, S *__restrict__ out,
                                                               const Geom g, int64_t nseg, S coef) {
+    overlap_wait();
     using O = ops<S>;
     using V = vec16<S>;
     constexpr int K = V::n / NC;                 // elements per vector
@@ -652,6 +655,7 @@ __global__ void __launch_bounds__(256) stencil3d_march_kernel(const cpx<S> *__re
     __shared__ uint64_t s_bar[kMarchSlots];
     const int L = (int)g.L, N = (int)g.n, P = (int)g.p, VEC = (int)g.vec;
     const int tid = threadIdx.x;
+    overlap_wait();
     const int logL = g.logL, vsh = g.logVEC, vmask = VEC - 1, bl = (int)g.b - 1;
     // slot: halo row above, TY rows, halo row below; then the edge area [side][row][VEC]
     const int slotE = (TY + 2) * L + 2 * TY * VEC;
@@ -869,9 +873,15 @@ static cudaError_t launch_march_ty(const zm_plan_s *p, const S *in, S *out, S co
         if (e != cudaSuccess) return e;
         attr_done[dev] = 1;
     }
-    int per_sm = 0, sms = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    // resident CTAs per SM of the calling thread's last shape (the query costs as much as the launch)
+    thread_local struct { int dev; size_t smem; int per_sm, sms; } occ = {-1, 0, 0, 0};
+    if (occ.dev != dev || occ.smem != smem) {
+        int per = 0, n = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, smem)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        occ = {dev, smem, per, n};
+    }
+    const int per_sm = occ.per_sm, sms = occ.sms;
     if (per_sm < 1) return cudaErrorNotSupported;
     const int64_t cols = g.p * g.p, tiles = g.L / TY;
     // depth chunks: at least four waves of resident CTAs (a short tail), each chunk walking
@@ -880,10 +890,9 @@ static cudaError_t launch_march_ty(const zm_plan_s *p, const S *in, S *out, S co
     int64_t chunks = 1;
     while (cols * tiles * chunks < 4 * (int64_t)per_sm * sms && g.n / (chunks * 2) >= 16) chunks *= 2;
     const int zsteps = (int)(g.n / chunks);
-    kern<<<(unsigned)(cols * tiles * chunks), 256, smem, st>>>(reinterpret_cast<const cpx<S> *>(in),
-                                                               reinterpret_cast<cpx<S> *>(out), g, zsteps, coef,
-                                                               p->dev_err);
-    return cudaGetLastError();
+    return launch_overlapped(kern, (unsigned)(cols * tiles * chunks), 256, smem, st,
+                             reinterpret_cast<const cpx<S> *>(in), reinterpret_cast<cpx<S> *>(out), g, zsteps, coef,
+                             p->dev_err);
 }
 template <typename S>
 static cudaError_t launch_march(const zm_plan_s *p, const S *in, S *out, S coef, cudaStream_t st) {
@@ -911,12 +920,15 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
     // 1 / (12 delta) for the FP32 derivatives (delta = coef for dx / dy, coef2 for ST_ALL)
     const double dl = op == ST_ALL ? coef2 : coef;
     const S rd = (S)(1.0 / (12.0 * dl));
+    cudaError_t e = cudaSuccess;
     if (p->g.dim == 2) {
         auto blocks = [&](int ry) { return (unsigned)((nvec / ry + threads - 1) / threads); };
 #define ZM_ROWS(OP, RY) \
-    stencil_rows_kernel<S, NC, OP, RY><<<blocks(RY), threads, 0, st>>>(i, o, o2, o3, p->g, nvec / RY, c, c2, rd)
+    e = launch_overlapped(stencil_rows_kernel<S, NC, OP, RY>, blocks(RY), threads, 0, st, i, o, o2, o3, p->g,  \
+                          nvec / RY, c, c2, rd)
 #define ZM_ROWSB(OP, RY, MB) \
-    stencil_rowsb_kernel<S, NC, OP, RY, MB><<<blocks(RY), threads, 0, st>>>(i, o, o2, o3, p->g, nvec / RY, c, c2, rd)
+    e = launch_overlapped(stencil_rowsb_kernel<S, NC, OP, RY, MB>, blocks(RY), threads, 0, st, i, o, o2, o3,   \
+                          p->g, nvec / RY, c, c2, rd)
         if constexpr (sizeof(S) == 8) {
             // FP64, us at N = 4096, P = 4, B = 64, c128 / real field.  dy, whose outputs share
             // rows: four rows of a B-row block per thread (118 / 60 with one row, 96 / 52 with
@@ -943,13 +955,13 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
         } else if (p->g.b == 2 && op == ST_ALL) {
             ZM_ROWSB(ST_ALL, 2, 4);
         } else if (op == ST_LAPLACE)
-            stencil_kernel<S, NC, ST_LAPLACE, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+            e = launch_overlapped(stencil_kernel<S, NC, ST_LAPLACE, 2>, grid, threads, 0, st, i, o, o2, o3, p->g, nvec, c, c2, rd);
         else if (op == ST_DX)
-            stencil_kernel<S, NC, ST_DX, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+            e = launch_overlapped(stencil_kernel<S, NC, ST_DX, 2>, grid, threads, 0, st, i, o, o2, o3, p->g, nvec, c, c2, rd);
         else if (op == ST_DY)
-            stencil_kernel<S, NC, ST_DY, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+            e = launch_overlapped(stencil_kernel<S, NC, ST_DY, 2>, grid, threads, 0, st, i, o, o2, o3, p->g, nvec, c, c2, rd);
         else
-            stencil_kernel<S, NC, ST_ALL, 2><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+            e = launch_overlapped(stencil_kernel<S, NC, ST_ALL, 2>, grid, threads, 0, st, i, o, o2, o3, p->g, nvec, c, c2, rd);
 #undef ZM_ROWS
 #undef ZM_ROWSB
     } else {
@@ -965,13 +977,13 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
         if (vline % (32 * RX) == 0 && p->g.vec % K == 0) {
             const int64_t nseg = nvec / (32 * RX);
             const unsigned gs = (unsigned)((nseg * 32 + threads - 1) / threads);
-            stencil3d_lines_kernel<S, NC, RX><<<gs, threads, 0, st>>>(i, o, p->g, nseg, c);
+            e = launch_overlapped(stencil3d_lines_kernel<S, NC, RX>, gs, threads, 0, st, i, o, p->g, nseg, c);
         } else {
-            stencil_kernel<S, NC, ST_LAPLACE, 3><<<grid, threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c, c2, rd);
+            e = launch_overlapped(stencil_kernel<S, NC, ST_LAPLACE, 3>, grid, threads, 0, st, i, o, o2, o3, p->g, nvec, c, c2, rd);
         }
     }
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_stencil(const zm_plan_s *p, int op, bool real_field, const void *in, void *out,
