@@ -378,8 +378,8 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
         const int lgs[2] = {lg, dtype == ZM_C128 && ltl == 0 ? 1 : lg};
         for (int o = 0; o < 2; o++)
             for (int a = 0; a < dim; a++)
-                P->axis[o][a] = zm::axis_map(g, kinds[dim - 2][a], dtype, ltl, lp, le, lgs[o]);
-        zm::axis_twiddles(g, le, &exps);
+                P->axis[o][a] = zm::axis_map(g, kinds[dim - 2][a], dtype, ltl, lp, zm::axis_digits(g.logN, le), lgs[o]);
+        zm::axis_twiddles(g, zm::axis_digits(g.logN, le), &exps);
     }
     if (flags & ZM_FLAG_HOST_ONLY) {
         *plan = P;
@@ -388,7 +388,8 @@ int zm_plan_create(zm_plan *plan, int dim, int64_t n, int64_t b, int64_t p, int 
     const int64_t entries = 2 * n + g.vec + g.m + 1 + (int64_t)exps.size();   // + one 16-byte slot for the error word
     std::vector<unsigned char> host((size_t)entries * 16);
     // w_N^m once; the other tables are subsets of it (VEC, M divide N, all powers of two)
-    std::vector<double> w((size_t)(2 * n));
+    std::vector<double> &w = P->roots;
+    w.resize((size_t)(2 * n));
     zm::unit_roots(n, w.data());
     auto put = [&](int64_t slot, int64_t m, bool fp64 = false) {
         unsigned char *at = host.data() + (size_t)slot * 16;

@@ -70,17 +70,18 @@ void order_lanes(std::vector<Bit> &v, int nthread, int phase, int banks, int lin
 }
 }  // namespace
 
-AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, int le, int lg) {
+// `lrs`: log2 radices of the digits, high to low
+AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, const std::vector<int> &lrs, int lg) {
     AxisMap m;
     memset(&m, 0, sizeof m);
     m.ltl = ltl;
     m.lp = lp;
-    m.le = le;
+    m.le = *std::max_element(lrs.begin(), lrs.end());
     // complex64 moves 16-byte pairs of the vector side: its lowest address bit must lie in
     // the tile, which an interleave wider than the tile's lines would break
     if (dtype != 0) lg = std::min(lg, ltl);
     m.lg = g.dim == 2 ? std::min(lg, g.logL) : 0;
-    const int ln = g.logN, lnt = ln + ltl - lp, nst = axis_stages(ln, le), lr = axis_lr(ln, le, nst - 1);
+    const int ln = g.logN, lnt = ln + ltl - lp, nst = (int)lrs.size(), lr = lrs[nst - 1];
     const LineAddr z = line_addr(g, kind, 0, m.lg);
     std::vector<Bit> va, fa;
     for (int j = 0; j < ltl; j++) {
@@ -105,9 +106,9 @@ AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, int le, in
         else w = z.f_lg ? (pos >> z.f_lg) * z.f_hi : pos * z.f_pos;
         // k bit -> index bit: stage s holds k bits [o, o + lr_s) at i bits [sh_s, ...)
         int o = 0, s = 0;
-        while (b >= o + axis_lr(ln, le, s)) o += axis_lr(ln, le, s++);
+        while (b >= o + lrs[s]) o += lrs[s++];
         if (s == nst - 1) digit.push_back(w);
-        else fa.push_back({w, ltl + axis_sh(ln, le, s) + b - o});
+        else fa.push_back({w, ltl + (ln - o - lrs[s]) + b - o});
     }
     auto by_addr = [](const Bit &x, const Bit &y) { return x.a < y.a; };
     std::sort(va.begin(), va.end(), by_addr);
@@ -131,16 +132,22 @@ AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, int le, in
     return m;
 }
 
+std::vector<int> axis_digits(int ln, int le) {
+    std::vector<int> lrs;
+    for (int s = 0; s < axis_stages(ln, le); s++) lrs.push_back(axis_lr(ln, le, s));
+    return lrs;
+}
+
 // exponent e of every table entry (w_N^e): stage s, row k, column v -> w_{N_s}^{k v}
-int64_t axis_twiddles(const Geom &g, int le, std::vector<int64_t> *exps) {
-    const int ln = g.logN, nst = axis_stages(ln, le);
-    for (int s = 0; s + 1 < nst; s++) {
-        const int lr = axis_lr(ln, le, s), sh = axis_sh(ln, le, s);
+void axis_twiddles(const Geom &g, const std::vector<int> &lrs, std::vector<int64_t> *exps) {
+    int sh = g.logN;
+    for (size_t s = 0; s + 1 < lrs.size(); s++) {
+        const int ln = g.logN, lr = lrs[s];
+        sh -= lr;
         for (int64_t k = 0; k < 1 << lr; k++)
             for (int64_t v = 0; v < 1 << sh; v++)
                 exps->push_back(((k * v) << (ln - lr - sh)) & (g.n - 1));
     }
-    return (int64_t)exps->size();
 }
 
 void unit_roots(int64_t n, double *w) {
@@ -163,9 +170,7 @@ void twiddle_store(int dtype, double c, double s, void *at) {
     }
 }
 
-void twiddle_entries(int64_t n, int dtype, const std::vector<int64_t> &exps, void *out) {
-    std::vector<double> w((size_t)(2 * n));
-    unit_roots(n, w.data());
+void twiddle_entries(const std::vector<double> &w, int dtype, const std::vector<int64_t> &exps, void *out) {
     for (size_t i = 0; i < exps.size(); i++)
         twiddle_store(dtype, w[2 * exps[i]], w[2 * exps[i] + 1], static_cast<unsigned char *>(out) + 16 * i);
 }

@@ -44,6 +44,18 @@ constexpr int axis_tw(int ln, int le, int s) {
     for (int q = 0; q < s; q++) o += 1 << (axis_lr(ln, le, q) + axis_sh(ln, le, q));
     return o;
 }
+// The same as a trait of AxisPass, which other digit lists replace (zm_batch_exact.cu):
+// row(s): log2 entries per row of stage s's table; col<s>(iv): the entry of a thread whose
+// index bits outside the digit are iv (those above it, then the lower digits v)
+template <int LN, int LE> struct AxisDigits {
+    static constexpr int NST = axis_stages(LN, LE);
+    static constexpr int lr(int s) { return axis_lr(LN, LE, s); }
+    static constexpr int sh(int s) { return axis_sh(LN, LE, s); }
+    static constexpr int row(int s) { return sh(s); }
+    static constexpr int tw(int s) { return axis_tw(LN, LE, s); }
+    template <int s> static __host__ __device__ constexpr int col(int iv) { return iv & ((1 << sh(s)) - 1); }
+    static constexpr int r0(int) { return 1; }   // first row whose entries are not all 1
+};
 __host__ __device__ constexpr int axis_slot(int i) { return i + (i >> 4) + (i >> 8) + (i >> 12); }
 
 // LP: log2 points per thread; LE: log2 of the largest digit (LE <= LP)
@@ -126,10 +138,12 @@ template <int NB, typename W> ZM_DEV int axis_bits(int x, W &&w) {
     return o;
 }
 
-template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = AxisParamMap> struct AxisPass {
+template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = AxisParamMap,
+          typename D = AxisDigits<LN, LE>>
+struct AxisPass {
     using C = cpx<T>;
     using CF = AxisCfg<T, LN, LTL, LP, LE>;
-    static constexpr int NT = CF::NT, LNT = CF::LNT, NST = CF::NST, EPT = 1 << LP;
+    static constexpr int NT = CF::NT, LNT = CF::LNT, NST = D::NST, EPT = 1 << LP;
     static constexpr int DIR = INV ? 1 : -1;
     // codelet constants as hi + lo pairs: the 45 degree ones, and complex64's 32-point level.
     // Round trip against FP64, without and with: 3D N = 256 c64 2.8e-7 / 2.4e-7 (at every
@@ -173,7 +187,7 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
             prefetch(in + axis_bits<LP>(r, [&](int b) { return m.va(LNT + b); }));
     }
     static ZM_DEV void prefetch_edge(const C *gm, const MAP &m, int tid) {
-        constexpr int lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, LU = LP - lr;
+        constexpr int lr = D::lr(NST - 1), R = 1 << lr, LU = LP - lr;
         gm += axis_bits<LNT>(tid, [&](int b) { return m.fa(b); });
 #pragma unroll
         for (int u = 0; u < 1 << LU; u++)
@@ -204,7 +218,7 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
     // The stage next to the frequency side (the last one forward, the first inverse): units
     // in frequency-side order, global memory at `gm` on that side.
     template <bool BAR = false> static ZM_DEV void edge_stage(C *S, C *gm, const MAP &m, int tid, bool scl, T sr, T si) {
-        constexpr int lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, LU = LP - lr;
+        constexpr int lr = D::lr(NST - 1), R = 1 << lr, LU = LP - lr;
         gm += axis_bits<LNT>(tid, [&](int b) { return m.fa(b); });
         S += axis_bits<LNT>(tid, [&](int b) { return m.fs(b); });
         auto ga = [&](int r) { return axis_bits<lr>(r, [&](int b) { return m.fr(b); }); };
@@ -236,20 +250,20 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
     // one `h` differ in the highest line bits only and share their twiddles.  TM: the
     // twiddles come from the thread's share of tensor memory at `tm`, else from the table.
     template <int s> struct Inner {
-        static constexpr int lr = axis_lr(LN, LE, s), sh = axis_sh(LN, LE, s), shp = sh + LTL, R = 1 << lr, LU = LP - lr;
+        static constexpr int lr = D::lr(s), sh = D::sh(s), shp = sh + LTL, R = 1 << lr, LU = LP - lr;
         static constexpr int LUT = LTL < LU ? LTL : LU, LT0 = LTL - LUT, HI = 1 << (LU - LUT), LO = 1 << LUT;
         static ZM_DEV int iv(int tid, int h) { return (tid + h * NT) >> LT0; }   // (bits above the digit, v)
-        static ZM_DEV int v(int tid, int h) { return iv(tid, h) & ((1 << sh) - 1); }
+        static ZM_DEV int col(int tid, int h) { return D::template col<s>(iv(tid, h)); }   // of the twiddle table
     };
     template <int s, bool TM> static ZM_DEV void inner_stage(C *S, const tw<T> *tb, uint32_t tm, int tid) {
         using G = Inner<s>;
         constexpr int R = G::R, HI = G::HI, LO = G::LO, LT0 = G::LT0, sh = G::sh, shp = G::shp, lr = G::lr;
         constexpr bool MEM = TM && s >= CF::TM0;
-        tb += axis_tw(LN, LE, s);
+        tb += D::tw(s);
 #pragma unroll
         for (int h = 0; h < HI; h++) {
-            const int iv = G::iv(tid, h), v = G::v(tid, h);
-            const int i = ((iv >> sh) << (sh + lr)) | v;
+            const int iv = G::iv(tid, h);
+            const int i = ((iv >> sh) << (sh + lr)) | (iv & ((1 << sh) - 1));
             const int slot = axis_slot((i << LTL) | ((tid + h * NT) & ((1 << LT0) - 1)));
             C x[LO][R];
 #pragma unroll
@@ -276,8 +290,8 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
                     }
                 } else {
 #pragma unroll
-                    for (int r = 1; r < R; r++) {
-                        const tw<T> w = ldtw(tb, (r << sh) + v);
+                    for (int r = D::r0(s); r < R; r++) {
+                        const tw<T> w = ldtw(tb, (r << D::row(s)) + G::col(tid, h));
 #pragma unroll
                         for (int q = 0; q < LO; q++) x[q][r] = twmul<INV>(x[q][r], w);
                     }
@@ -299,7 +313,7 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
         if constexpr (s < NST - 1) {
             using G = Inner<s>;
             constexpr int NE = (G::R - 1) * G::HI;
-            const tw<T> *t = tb + axis_tw(LN, LE, s);
+            const tw<T> *t = tb + D::tw(s);
 #pragma unroll 1
             for (int c = 0; c < (NE + 3) / 4; c++) {
                 uint32_t w16[16];
@@ -307,7 +321,7 @@ template <typename T, int LN, int LTL, int LP, int LE, bool INV, typename MAP = 
                 for (int e = 0; e < 4; e++) {
                     const int n = 4 * c + e < NE ? 4 * c + e : NE - 1;
                     const int h = n / (G::R - 1), r = n % (G::R - 1) + 1;
-                    const tw<T> w = ldtw(t, (r << G::sh) + G::v(tid, h));
+                    const tw<T> w = ldtw(t, (r << D::row(s)) + G::col(tid, h));
                     memcpy(w16 + 4 * e, &w, 16);
                 }
                 tmem_st16(tm + CF::tm_at(s) + 16 * c, w16);

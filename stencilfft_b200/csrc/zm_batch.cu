@@ -7,14 +7,15 @@
 // generator ...), with a grid barrier between steps.  Inside a pass step the work items
 // are tiles of TL lines of one field, TL * N = a fixed number of points per tile, so the
 // same CTA shape serves every N; a tile's field comes from a binary search over the
-// fields' first tile numbers.  Two kernels hold the tile code: batch_axis_kernel on the axis
-// pass sized by N alone (zm_batch_axis.cuh), and batch_kernel on the VEC x M split of
-// zm_tile.cuh for the complex64 Poisson call with a residual (see zm_batch_poisson) and for
-// fields below N = 64.
-#include <cuda/atomic>
+// fields' first tile numbers.  Three kernels hold the tile code: batch_axis_kernel on the
+// axis pass sized by N alone (zm_batch_axis.cuh); batch_exact_kernel (zm_batch_exact.cu) for
+// the complex64 Poisson call with a residual, which keeps the rounding of the VEC x M split
+// (see zm_batch_poisson); and batch_kernel on that split (zm_tile.cuh) for those calls where
+// a field's VEC is 1 or above 16, and for fields below N = 64.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -22,105 +23,12 @@
 #include <tuple>
 #include <vector>
 
-#include "zm_index.cuh"
-#include "zm_internal.h"
+#include "zm_batch.cuh"
 #include "zm_batch_axis.cuh"
 #include "zm_tile.cuh"
 #include "zmodel_b200.h"
 
 namespace zm {
-
-constexpr int kBatchThreads = 256;
-constexpr int kMaxSteps = 6;
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;   // 2 s
-
-struct BatchField {
-    Geom g;
-    int64_t off;       // element offset in a batch buffer
-    int64_t tile0;     // first tile of this field in a pass step's tile sequence
-    const void *twN;   // the field plan's twiddle table w_N^m (tw<T> entries)
-    const AxisMap *ax; // weight tables of the x and y passes (batches on the axis tiles)
-    const void *twx;   // their stage twiddles
-    int T;             // lines per tile
-    int nst_vec, nst_m;
-    int rad_vec[8], rad_m[8];
-};
-
-enum BatchOp : int {
-    BOP_X_FWD = 0,     // x pass forward: real layout -> REPACK layout
-    BOP_Y_FWD = 1,     // y pass forward: REPACK layout -> reciprocal layout
-    BOP_Y_INV = 2,     // y pass inverse
-    BOP_X_INV = 3,     // x pass inverse (scale 1/N^2 when step.scale)
-    BOP_Y_POISSON = 4, // y pass forward, divide by -|k|^2, y pass inverse (in place)
-    BOP_RESIDUAL = 5,  // out = Lap(in) / h^2 - aux (5-point, periodic)
-    BOP_FILL = 6,      // out = generator(kind, seed + field) in the real layout
-    BOP_NOP = 7        // nothing (barrier probe)
-};
-
-struct BatchStep {
-    int op;
-    int kind;          // BOP_FILL: zm_field_kind
-    int scale;         // BOP_X_INV: apply 1/N^2
-    const void *in;
-    void *out;
-    const void *aux;
-    double a;          // BOP_Y_POISSON: 2 pi / length; BOP_RESIDUAL: 1 / length
-    uint64_t seed;
-};
-
-struct BatchParams {
-    const BatchField *fields;
-    const int *tile_field;   // field of each tile (batches on the axis tiles)
-    int nfields;
-    int64_t tiles;
-    int nsteps;
-    BatchStep step[kMaxSteps];
-    unsigned *bar;     // [0] arrivals, [1] generation
-    int *abort;        // this launch only: set by a barrier that timed out, the others give up
-    int *err;          // sticky: set by a barrier that timed out, read and cleared by zm_batch_status
-    unsigned missing;  // arrivals a barrier waits for beyond the grid (0; > 0 only in the probe)
-};
-
-ZM_DEV unsigned long long globaltimer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid-wide barrier of a cooperative launch (all CTAs resident).  Sense by generation
-// count; the last CTA to arrive resets the arrival count and releases the generation.
-// A wait longer than kBarrierTimeoutNs, or an abort already raised by another CTA of
-// this launch, makes every waiting CTA give up: returns false and the kernel returns.
-// A timeout also raises the sticky error word that zm_batch_status reports; the abort
-// word is cleared before every launch, so one timeout ends only its own launch.
-ZM_DEV bool grid_barrier(unsigned *bar, unsigned nblocks, int *abort, int *err, int *s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        cuda::atomic_ref<unsigned, cuda::thread_scope_device> cnt(bar[0]), gen(bar[1]);
-        cuda::atomic_ref<int, cuda::thread_scope_device> flag(*abort), sticky(*err);
-        const unsigned g0 = gen.load(cuda::memory_order_acquire);
-        if (cnt.fetch_add(1u, cuda::memory_order_acq_rel) == nblocks - 1) {
-            cnt.store(0u, cuda::memory_order_relaxed);
-            gen.fetch_add(1u, cuda::memory_order_release);
-        } else {
-            const unsigned long long t0 = globaltimer_ns();
-            while (gen.load(cuda::memory_order_acquire) == g0) {
-                if (flag.load(cuda::memory_order_relaxed) != 0 ||
-                    globaltimer_ns() - t0 > kBarrierTimeoutNs) {
-                    flag.store(1, cuda::memory_order_relaxed);
-                    sticky.store(1, cuda::memory_order_relaxed);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(128);
-            }
-        }
-        *s_ok = ok;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
 
 // largest f with fields[f].tile0 <= tile
 ZM_DEV int field_of_tile(const BatchField *fields, int nfields, int64_t tile) {
@@ -131,15 +39,6 @@ ZM_DEV int field_of_tile(const BatchField *fields, int nfields, int64_t tile) {
         else hi = mid - 1;
     }
     return lo;
-}
-
-// global (row, col) -> element of the real layout (inverse of real_gidx, 2D)
-ZM_DEV int64_t real_elem(int64_t gr, int64_t gc, const Geom &g) {
-    const int64_t rid = (gr >> g.logB) & (g.p - 1);
-    const int64_t lr = ((gr >> (g.logB + g.logP)) << g.logB) + (gr & (g.b - 1));
-    const int64_t cid = (gc >> g.logB) & (g.p - 1);
-    const int64_t pos = ((gc & (g.b - 1)) << g.logVEC) + (gc >> (g.logB + g.logP));
-    return (((rid << g.logP) + cid) << (2 * g.logL)) + (lr << g.logL) + pos;
 }
 
 // Both sub-transforms of a tile: compile-time-sized stages (LMC = log2 M) for the
@@ -260,94 +159,6 @@ __device__ __noinline__ void batch_tile(int op, bool scale, double a, const Batc
     }
 }
 
-// One tile of the residual step, out = Lap_h(in) - rhs over elements [e0, e0 + TP) of a
-// field (5-point, periodic, h = length / N, a = 1 / length); its own function so that its
-// registers do not weigh on the rest of the persistent kernel.
-template <typename T, int TP>
-__device__ __noinline__ void residual_tile(const Geom &g, double a, const cpx<T> *in, const cpx<T> *rhs, cpx<T> *out,
-                                           int64_t e0, int nthr, int tid) {
-    const T inv_h2 = (T)((double)g.n * a * (double)g.n * a);
-    const int64_t m = g.n - 1;
-    auto resid = [&](const cpx<T> &up, const cpx<T> &dn, const cpx<T> &lf, const cpx<T> &rt,
-                     const cpx<T> &c, const cpx<T> &r) -> cpx<T> {
-        const T lx = up.x + dn.x + lf.x + rt.x - (T)4 * c.x;
-        const T ly = up.y + dn.y + lf.y + rt.y - (T)4 * c.y;
-        return {lx * inv_h2 - r.x, ly * inv_h2 - r.y};
-    };
-    if constexpr (sizeof(T) == 4) {
-        // Pairs (e, e + 1), e even: the two share rank and row (L is even), so
-        // their up / down neighbours are again two adjacent elements, and so
-        // are left / right except at a block edge.  Adjacent 16-byte-aligned
-        // pairs move as one 16-byte access, anything else element by element.
-        auto ld2 = [](const cpx<T> *p0, const cpx<T> *p1, cpx<T> &v0, cpx<T> &v1) {
-            if (p1 == p0 + 1 && ((uintptr_t)p0 & 15) == 0) {
-                const float4 q = __ldg(reinterpret_cast<const float4 *>(p0));
-                v0 = {q.x, q.y};
-                v1 = {q.z, q.w};
-            } else {
-                v0 = ldg(p0);
-                v1 = ldg(p1);
-            }
-        };
-        // Inside a rank's B x B block (in-block column j = pos >> log VEC and
-        // row lr mod B both off the block's edges) the four neighbours of the
-        // pair sit in the same rank at -L, +L (rows) and -VEC, +VEC (columns:
-        // the next global column is the next in-block column of the same
-        // block cycle), adjacent pairs again when VEC >= 2.
-        const bool fast = g.logVEC >= 1 &&
-                          (((uintptr_t)in | (uintptr_t)rhs | (uintptr_t)out) & 15) == 0;
-        // the geometry in registers (g lives in shared memory; a field holds < 2^31 elements)
-        const int iL = (int)g.L, iV = (int)g.vec, bm = (int)g.b - 1, logL = g.logL, logV = g.logVEC;
-        auto q4 = [](const cpx<T> *q) { return __ldg(reinterpret_cast<const float4 *>(q)); };
-        for (int i = tid; i < TP / 2; i += nthr) {
-            const int64_t e = e0 + 2 * i;
-            const int pos = (int)e & (iL - 1), lr = ((int)e >> logL) & (iL - 1);
-            const int j = pos >> logV, rb = lr & bm;
-            if (fast && j > 0 && j < bm && rb > 0 && rb < bm) {
-                const cpx<T> *pc = in + e;
-                const float4 up = q4(pc - iL), dn = q4(pc + iL), lf = q4(pc - iV), rt = q4(pc + iV);
-                const float4 cc = q4(pc), rr = q4(rhs + e);
-                const cpx<T> o0 = resid({up.x, up.y}, {dn.x, dn.y}, {lf.x, lf.y}, {rt.x, rt.y},
-                                        {cc.x, cc.y}, {rr.x, rr.y});
-                const cpx<T> o1 = resid({up.z, up.w}, {dn.z, dn.w}, {lf.z, lf.w}, {rt.z, rt.w},
-                                        {cc.z, cc.w}, {rr.z, rr.w});
-                *reinterpret_cast<float4 *>(out + e) = make_float4(o0.x, o0.y, o1.x, o1.y);
-                continue;
-            }
-            const int64_t gi0 = real_gidx(e, g), gc1 = real_gidx(e + 1, g) & m;
-            const int64_t gr = gi0 >> g.logN, gc0 = gi0 & m;
-            const int64_t au = real_elem((gr - 1) & m, gc0, g), ad = real_elem((gr + 1) & m, gc0, g);
-            cpx<T> up0, up1, dn0, dn1, lf0, lf1, rt0, rt1, c0, c1, r0, r1;
-            ld2(in + au, in + au + 1, up0, up1);
-            ld2(in + ad, in + ad + 1, dn0, dn1);
-            ld2(in + real_elem(gr, (gc0 - 1) & m, g), in + real_elem(gr, (gc1 - 1) & m, g), lf0, lf1);
-            ld2(in + real_elem(gr, (gc0 + 1) & m, g), in + real_elem(gr, (gc1 + 1) & m, g), rt0, rt1);
-            ld2(in + e, in + e + 1, c0, c1);
-            ld2(rhs + e, rhs + e + 1, r0, r1);
-            const cpx<T> o0 = resid(up0, dn0, lf0, rt0, c0, r0);
-            const cpx<T> o1 = resid(up1, dn1, lf1, rt1, c1, r1);
-            cpx<T> *po = out + e;
-            if (((uintptr_t)po & 15) == 0) {
-                *reinterpret_cast<float4 *>(po) = make_float4(o0.x, o0.y, o1.x, o1.y);
-            } else {
-                po[0] = o0;
-                po[1] = o1;
-            }
-        }
-    } else {
-        for (int i = tid; i < TP; i += nthr) {
-            const int64_t e = e0 + i;
-            const int64_t gi = real_gidx(e, g);
-            const int64_t gr = gi >> g.logN, gc = gi & m;
-            const cpx<T> up = ldg(in + real_elem((gr - 1) & m, gc, g));
-            const cpx<T> dn = ldg(in + real_elem((gr + 1) & m, gc, g));
-            const cpx<T> lf = ldg(in + real_elem(gr, (gc - 1) & m, g));
-            const cpx<T> rt = ldg(in + real_elem(gr, (gc + 1) & m, g));
-            out[e] = resid(up, dn, lf, rt, ldg(in + e), ldg(rhs + e));
-        }
-    }
-}
-
 template <typename T, int EPT>
 __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchParams bp) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -397,7 +208,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPara
                 }
                 const cpx<T> *in = reinterpret_cast<const cpx<T> *>(S.in) + sf.off;
                 const cpx<T> *rhs = reinterpret_cast<const cpx<T> *>(S.aux) + sf.off;
-                residual_tile<T, TP>(sf.g, S.a, in, rhs, out, e0, nthr, tid);
+                residual_tile<T, TP>(g, S.a, in, rhs, out, e0, s, tid);
             }
             continue;
         }
@@ -486,8 +297,8 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(T) == 4 ? 4 : 2) batch_a
             const cpx<T> *in = reinterpret_cast<const cpx<T> *>(S.in) + f.off;
             cpx<T> *out = reinterpret_cast<cpx<T> *>(S.out) + f.off;
             if (op == BOP_RESIDUAL) {
-                residual_tile<T, TP>(g, S.a, in, reinterpret_cast<const cpx<T> *>(S.aux) + f.off, out, sub * TP,
-                                     kBatchThreads, threadIdx.x);
+                residual_tile<T, TP>(g, S.a, in, reinterpret_cast<const cpx<T> *>(S.aux) + f.off, out, sub * TP, s,
+                                     threadIdx.x);
                 continue;
             }
             if (op == BOP_FILL) {
@@ -513,14 +324,16 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(T) == 4 ? 4 : 2) batch_a
     }
 }
 
-// kernel, dynamic shared memory and opt-in of a batch on the axis tiles or the runtime-sized ones
+// kernel and dynamic shared memory of a call
+enum BatchTiles : int { TILES_SPLIT = 0, TILES_AXIS = 1, TILES_EXACT = 2 };
 struct BatchKernel {
-    void (*fn)(const BatchParams);
+    BatchFn fn;
     size_t smem;
 };
-static BatchKernel batch_kernel_of(int dtype, bool axis) {
+static BatchKernel batch_kernel_of(int dtype, int tiles) {
     constexpr size_t slots = axis_slot((1 << kBatchTileLog) - 1) + 1;
-    if (axis) return dtype == 0 ? BatchKernel{batch_axis_kernel<double>, slots * 16}
+    if (tiles == TILES_EXACT) return BatchKernel{batch_exact_fn(), slots * 8};
+    if (tiles == TILES_AXIS) return dtype == 0 ? BatchKernel{batch_axis_kernel<double>, slots * 16}
                                 : BatchKernel{batch_axis_kernel<float>, slots * 8};
     return dtype == 0 ? BatchKernel{batch_kernel<double, 8>, kBatchThreads * 8 * 16}
                       : BatchKernel{batch_kernel<float, 16>, kBatchThreads * 16 * 8};
@@ -567,7 +380,8 @@ struct zm_batch_s {
     std::vector<int> field_plan;
     zm::BatchField *d_fields = nullptr;
     bool axis = false;                     // every field fits the axis tiles (zm_batch_axis.cuh)
-    int axis_grid = 0;
+    bool exact = false;                    // every field fits the tiles of zm_batch_exact.cu
+    int axis_grid = 0, exact_grid = 0;
     int64_t axis_tiles = 0;
     const zm::BatchField *axis_fields = nullptr;   // the fields as the axis tiles count them
     const int *tile_field = nullptr;
@@ -595,22 +409,24 @@ bool overlap_b(const void *a, const void *b, size_t bytes) {
     return x < y + bytes && y < x + bytes;
 }
 
-// `axis`: on the axis tiles when every field fits them
-int launch(zm_batch b, const zm::BatchStep *steps, int nsteps, void *stream, bool axis, unsigned missing = 0) {
-    axis = axis && b->axis;
+// `tiles`: the kernel asked for; batches whose fields do not all fit it run the split tiles
+int launch(zm_batch b, const zm::BatchStep *steps, int nsteps, void *stream, int tiles, unsigned missing = 0) {
+    if ((tiles == zm::TILES_AXIS && !b->axis) || (tiles == zm::TILES_EXACT && !b->exact)) tiles = zm::TILES_SPLIT;
+    const bool split = tiles == zm::TILES_SPLIT;
     zm::BatchParams bp = {};
     bp.missing = missing;
-    bp.fields = axis ? b->axis_fields : b->d_fields;
+    bp.fields = split ? b->d_fields : b->axis_fields;
     bp.tile_field = b->tile_field;
     bp.nfields = (int)b->fields.size();
-    bp.tiles = axis ? b->axis_tiles : b->tiles;
+    bp.tiles = split ? b->tiles : b->axis_tiles;
     bp.nsteps = nsteps;
     for (int i = 0; i < nsteps; i++) bp.step[i] = steps[i];
     bp.bar = b->d_sync;
     bp.abort = reinterpret_cast<int *>(b->d_sync + 2);
     bp.err = reinterpret_cast<int *>(b->d_sync + 3);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    cudaError_t e = zm::launch_batch(zm::batch_kernel_of(b->dtype, axis), bp, axis ? b->axis_grid : b->grid, st);
+    const int grid = split ? b->grid : tiles == zm::TILES_EXACT ? b->exact_grid : b->axis_grid;
+    cudaError_t e = zm::launch_batch(zm::batch_kernel_of(b->dtype, tiles), bp, grid, st);
     if (e != cudaSuccess)
         return zm::report_error(ZM_ERR_CUDA, "batch launch: %s (%s)", cudaGetErrorName(e), cudaGetErrorString(e));
     return ZM_OK;
@@ -630,22 +446,37 @@ int device_tables(zm_batch b) {
     size_t af_at = 0, tf_at = 0;
     std::vector<zm::BatchField> af;
     std::vector<size_t> map_at(b->plans.size()), tw_at(b->plans.size());
+    std::vector<std::array<size_t, 3>> ex_at(b->plans.size());   // exact tiles: tables, forward and inverse twiddles
     if (b->axis) {
         std::map<int, size_t> tw_of;   // log2 N -> stage twiddles
         for (size_t i = 0; i < b->plans.size(); i++) {
             const zm::Geom &g = b->plans[i]->g;
             const int ltl = zm::kBatchTileLog - g.logN, lg = std::min(ltl, 3);
-            const zm::AxisMap maps[2] = {zm::axis_map(g, zm::PASS_X2, b->dtype, ltl, zm::kBatchPtsLog, 4, lg),
-                                         zm::axis_map(g, zm::PASS_Y2, b->dtype, ltl, zm::kBatchPtsLog, 4, lg)};
+            const std::vector<int> lrs = zm::axis_digits(g.logN, 4);
+            const zm::AxisMap maps[2] = {zm::axis_map(g, zm::PASS_X2, b->dtype, ltl, zm::kBatchPtsLog, lrs, lg),
+                                         zm::axis_map(g, zm::PASS_Y2, b->dtype, ltl, zm::kBatchPtsLog, lrs, lg)};
             map_at[i] = reserve(sizeof maps);
             std::memcpy(&blob[map_at[i]], maps, sizeof maps);
             if (!tw_of.count(g.logN)) {
                 std::vector<int64_t> exps;
-                zm::axis_twiddles(g, 4, &exps);
+                zm::axis_twiddles(g, lrs, &exps);
                 tw_of[g.logN] = reserve(exps.size() * 16);
-                zm::twiddle_entries(g.n, b->dtype, exps, &blob[tw_of[g.logN]]);
+                zm::twiddle_entries(b->plans[i]->roots, b->dtype, exps, &blob[tw_of[g.logN]]);
             }
             tw_at[i] = tw_of[g.logN];
+            if (!b->exact) continue;
+            const std::vector<int> df = zm::batch_exact_digits(g, false), di = zm::batch_exact_digits(g, true);
+            const zm::AxisMap ex[3] = {zm::axis_map(g, zm::PASS_X2, b->dtype, ltl, zm::kBatchPtsLog, df, lg),
+                                       zm::axis_map(g, zm::PASS_Y2, b->dtype, ltl, zm::kBatchPtsLog, df, lg),
+                                       zm::axis_map(g, zm::PASS_X2, b->dtype, ltl, zm::kBatchPtsLog, di, lg)};
+            ex_at[i][0] = reserve(sizeof ex);
+            std::memcpy(&blob[ex_at[i][0]], ex, sizeof ex);
+            for (int inv = 0; inv < 2; inv++) {
+                std::vector<int64_t> exps;
+                zm::batch_exact_twiddles(g, inv, &exps);
+                ex_at[i][1 + inv] = reserve(exps.size() * 16);
+                zm::twiddle_entries(b->plans[i]->roots, b->dtype, exps, &blob[ex_at[i][1 + inv]]);
+            }
         }
         std::vector<int> tf;
         af = b->fields;
@@ -667,6 +498,10 @@ int device_tables(zm_batch b) {
         for (size_t i = 0; i < nf; i++) {
             af[i].ax = reinterpret_cast<const zm::AxisMap *>(d + map_at[b->field_plan[i]]);
             af[i].twx = d + tw_at[b->field_plan[i]];
+            const std::array<size_t, 3> &e = ex_at[b->field_plan[i]];
+            af[i].ex = b->exact ? reinterpret_cast<const zm::AxisMap *>(d + e[0]) : nullptr;
+            af[i].exf = b->exact ? d + e[1] : nullptr;
+            af[i].exi = b->exact ? d + e[2] : nullptr;
         }
         std::memcpy(&blob[af_at], af.data(), sizeof(zm::BatchField) * nf);
         b->axis_fields = reinterpret_cast<const zm::BatchField *>(d + af_at);
@@ -701,6 +536,7 @@ int zm_batch_create(zm_batch *batch, int nfields, const int64_t *n, const int64_
     // an axis tile is 4096 points of one field: N = 64 and up
     B->axis = true;
     for (int i = 0; i < nfields; i++) B->axis = B->axis && n[i] >= 64;
+    B->exact = B->axis && dtype == ZM_C64;
     for (int i = 0; i < nfields && rc == ZM_OK; i++) {
         if (n[i] < tile_pts / 64 || n[i] > tile_pts) {
             rc = zm::report_error(ZM_ERR_CONSTRAINT, "field %d: N=%lld outside the batch range [%lld, %lld]", i,
@@ -721,6 +557,7 @@ int zm_batch_create(zm_batch *batch, int nfields, const int64_t *n, const int64_
             pi = it->second;
         }
         const zm_plan_s *pl = B->plans[pi];
+        B->exact = B->exact && zm::batch_exact_fits(pl->g);
         zm::BatchField f = {};
         f.g = pl->g;
         f.off = B->elems;
@@ -735,9 +572,11 @@ int zm_batch_create(zm_batch *batch, int nfields, const int64_t *n, const int64_
         B->tiles += n[i] / f.T;
     }
     if (rc == ZM_OK) {
-        B->grid = zm::batch_grid(zm::batch_kernel_of(dtype, false), B->device);
-        if (B->axis) B->axis_grid = zm::batch_grid(zm::batch_kernel_of(dtype, true), B->device);
-        if (B->grid <= 0 || (B->axis && B->axis_grid <= 0)) rc = zm::report_error(ZM_ERR_CUDA, "batch kernel occupancy query failed");
+        B->grid = zm::batch_grid(zm::batch_kernel_of(dtype, zm::TILES_SPLIT), B->device);
+        if (B->axis) B->axis_grid = zm::batch_grid(zm::batch_kernel_of(dtype, zm::TILES_AXIS), B->device);
+        if (B->exact) B->exact_grid = zm::batch_grid(zm::batch_kernel_of(dtype, zm::TILES_EXACT), B->device);
+        if (B->grid <= 0 || (B->axis && B->axis_grid <= 0) || (B->exact && B->exact_grid <= 0))
+            rc = zm::report_error(ZM_ERR_CUDA, "batch kernel occupancy query failed");
     }
     if (rc == ZM_OK) rc = device_tables(B);
     if (rc == ZM_OK) {
@@ -795,7 +634,7 @@ int zm_batch_fill(zm_batch batch, void *data, int kind, uint64_t first_seed, voi
     s.kind = kind;
     s.out = data;
     s.seed = first_seed;
-    return launch(batch, &s, 1, stream, true);
+    return launch(batch, &s, 1, stream, zm::TILES_AXIS);
 }
 
 int zm_batch_forward(zm_batch batch, const void *in, void *out, void *stream) {
@@ -805,7 +644,7 @@ int zm_batch_forward(zm_batch batch, const void *in, void *out, void *stream) {
     zm::BatchStep s[2] = {};
     s[0].op = zm::BOP_X_FWD; s[0].in = in; s[0].out = out;
     s[1].op = zm::BOP_Y_FWD; s[1].in = out; s[1].out = out;
-    return launch(batch, s, 2, stream, true);
+    return launch(batch, s, 2, stream, zm::TILES_AXIS);
 }
 
 int zm_batch_inverse(zm_batch batch, const void *in, void *out, void *work, int normalise, void *stream) {
@@ -822,7 +661,7 @@ int zm_batch_inverse(zm_batch batch, const void *in, void *out, void *work, int 
     zm::BatchStep s[2] = {};
     s[0].op = zm::BOP_Y_INV; s[0].in = in; s[0].out = tmp;
     s[1].op = zm::BOP_X_INV; s[1].in = tmp; s[1].out = out; s[1].scale = normalise ? 1 : 0;
-    return launch(batch, s, 2, stream, true);
+    return launch(batch, s, 2, stream, zm::TILES_AXIS);
 }
 
 int zm_batch_poisson(zm_batch batch, const void *rhs, void *phi, void *residual, void *work, double length,
@@ -850,8 +689,9 @@ int zm_batch_poisson(zm_batch batch, const void *rhs, void *phi, void *residual,
     // The complex64 residual is a difference of nearly equal terms: it amplifies phi's
     // rounding by about 8 N / (2 pi)^2 (2e-5 of the residual at N = 256, 2e-4 at 2048), so
     // another order of the transforms' operations is another residual field.  Those calls
-    // keep the tiles, and the rounding, that they had.
-    return launch(batch, s, ns, stream, batch->dtype == ZM_C128 || !residual);
+    // keep the rounding of the VEC x M split, on its own tiles (zm_batch_exact.cu) or, for
+    // fields that these do not hold, on batch_kernel.
+    return launch(batch, s, ns, stream, batch->dtype == ZM_C128 || !residual ? zm::TILES_AXIS : zm::TILES_EXACT);
 }
 
 int zm_batch_status(zm_batch batch, int *device_error) {
@@ -877,7 +717,7 @@ int zm_batch_barrier_probe(zm_batch batch, int missing, void *stream) {
     zm::BatchStep s[2] = {};
     s[0].op = zm::BOP_NOP;
     s[1].op = zm::BOP_NOP;
-    return launch(batch, s, 2, stream, false, (unsigned)missing);
+    return launch(batch, s, 2, stream, zm::TILES_SPLIT, (unsigned)missing);
 }
 
 int zm_batch_autotune_b(int64_t n, int64_t p, int dtype, int count, int reps, int64_t *best_b, float *best_ms) {

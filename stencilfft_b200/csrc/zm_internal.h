@@ -65,14 +65,15 @@ int fused_inv_oop_c128(int logvec, int logm, int *vx, int *vy, int *lg, int *qin
 
 // zm_axis.cu: the axis pass sized by N alone
 bool axis_tile(const Geom &g, int dtype, int64_t total, int *ltl, int *lp, int *le);
-AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, int le, int lg);
-int64_t axis_twiddles(const Geom &g, int le, std::vector<int64_t> *exps);
+std::vector<int> axis_digits(int ln, int le);
+AxisMap axis_map(const Geom &g, int kind, int dtype, int ltl, int lp, const std::vector<int> &lrs, int lg);
+void axis_twiddles(const Geom &g, const std::vector<int> &lrs, std::vector<int64_t> *exps);
 // w_N^m = exp(-2 pi i m / N), m < N, generated in extended precision and rounded once
 void unit_roots(int64_t n, double *w);
 // one table entry (16 bytes, tw<T> of zm_common.cuh) from an FP64 value
 void twiddle_store(int dtype, double c, double s, void *at);
-// w_N^e for every e of exps
-void twiddle_entries(int64_t n, int dtype, const std::vector<int64_t> &exps, void *out);
+// w_N^e for every e of exps, from the plan's roots
+void twiddle_entries(const std::vector<double> &roots, int dtype, const std::vector<int64_t> &exps, void *out);
 cudaError_t launch_axis_pass(const AxisParams &p, int dtype, bool inv, int64_t nlines, cudaStream_t st);
 // zm_axis_<dtype>_<dir>.cu
 cudaError_t launch_axis_c64_fwd(const AxisParams &p, int64_t nlines, cudaStream_t st);

@@ -4,6 +4,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace zm {
 
 // Which axis pass of a transform a line kernel runs.  Every pass reads each
@@ -109,6 +111,7 @@ struct zm_plan_s {
     // the passes x, y, z on the kernel sized by N alone: [0] in place, [1] 2D forward with
     // a workspace (its own row interleave)
     zm::AxisMap axis[2][3];
+    std::vector<double> roots;   // w_N^m in FP64 (host)
     void *twx;        // its stage twiddles (inside the tables allocation)
     zm::PermMap perm[2][2];   // converters [reciprocal][to natural]
     void *own_work;   // ZM_FLAG_OWN_WORKSPACE: one field, used by transforms called with work = NULL

@@ -31,7 +31,7 @@ static Geom geom(int dim, int ln, int lb, int lp) {
 static void check(const Geom &g, int dtype, int kind, int ltl, int lp, int le, int lg) {
     const int ln = g.logN, lnt = ln + ltl - lp, nst = axis_stages(ln, le), lr = axis_lr(ln, le, nst - 1);
     const int64_t total = g.dim == 2 ? g.n * g.n : g.n * g.n * g.n, nblk = (total >> ln) >> ltl;
-    const AxisMap m = axis_map(g, kind, dtype, ltl, lp, le, lg);
+    const AxisMap m = axis_map(g, kind, dtype, ltl, lp, axis_digits(g.logN, le), lg);
     const int E = 1 << (ln + ltl);
     std::vector<int> index(axis_slot(E - 1) + 1, -1);
     for (int i = 0; i < E; i++) index[axis_slot(i)] = i;
