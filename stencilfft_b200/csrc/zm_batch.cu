@@ -274,7 +274,7 @@ __device__ __noinline__ void fill_tile(const Geom &g, int kind, uint64_t seed, c
 // 50 %.  32 + 32 + 24 + 8 complex64 fields of N = 256 .. 2048, P = 2, forward / inverse:
 // 986 / 884 -> 608 / 610 us at VEC = 4 (the split's compile-time tiles), 2221 / 2163 -> 608 /
 // 609 us at VEC = 16 (its runtime-sized tiles); 29 complex128 fields of N = 128 .. 1024,
-// P = 4: 237 / 233 -> 136 / 120 us.
+// P = 4: 237 / 233 -> 120 / 115 us (136 / 120 before odd steps walked back, walks_back).
 template <typename T>
 __global__ void __launch_bounds__(kBatchThreads, sizeof(T) == 4 ? 4 : 2) batch_axis_kernel(const BatchParams bp) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -286,12 +286,13 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(T) == 4 ? 4 : 2) batch_a
         const int op = bp.step[st].op;
         if (op == BOP_NOP) continue;
         const BatchStep &S = bp.step[st];
-        int64_t tile = blockIdx.x;
-        int fi = tile < bp.tiles ? __ldg(bp.tile_field + tile) : 0;
-        for (; tile < bp.tiles; tile += gridDim.x) {
+        const int ntiles = (int)bp.tiles, hop = walks_back(bp, st) ? -(int)gridDim.x : (int)gridDim.x;
+        int tile = hop < 0 ? ntiles - 1 - (int)blockIdx.x : (int)blockIdx.x;
+        int fi = tile < ntiles ? __ldg(bp.tile_field + tile) : 0;
+        for (; (unsigned)tile < (unsigned)ntiles; tile += hop) {
             const BatchField &f = bp.fields[fi];
             const int fcur = fi;
-            if (tile + gridDim.x < bp.tiles) fi = __ldg(bp.tile_field + tile + gridDim.x);
+            if ((unsigned)(tile + hop) < (unsigned)ntiles) fi = __ldg(bp.tile_field + tile + hop);
             const Geom &g = f.g;
             const int64_t sub = tile - f.tile0;   // of the field
             const cpx<T> *in = reinterpret_cast<const cpx<T> *>(S.in) + f.off;

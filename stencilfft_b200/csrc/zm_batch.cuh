@@ -104,6 +104,15 @@ ZM_DEV bool grid_barrier(unsigned *bar, unsigned nblocks, int *abort, int *err, 
     return *s_ok != 0;
 }
 
+// Odd steps walk the tiles from the last: what the step before wrote last is still in the L2
+// (126 MB), so a batch larger than that reads that part from there: 29 complex128 fields of
+// N = 128 .. 1024 (89 MB a buffer) forward 138 -> 120 us, Poisson call 302 -> 284 us; 16
+// complex64 fields of 1024^2 (134 MB) 354 -> 347 us; 96 fields (554 MB) unchanged.  From
+// buffers of 77 MB (four turns of the walk): below, everything is in the L2 either way, and a
+// CTA that keeps its tile is faster (300 complex128 fields of N = 64, Poisson call 70 us, 74
+// reversed).
+ZM_DEV bool walks_back(const BatchParams &bp, int step) { return (step & 1) && bp.tiles > 4 * (int64_t)gridDim.x; }
+
 // the kernel of the complex64 Poisson call with a residual (zm_batch_exact.cu)
 using BatchFn = void (*)(const BatchParams);
 BatchFn batch_exact_fn();

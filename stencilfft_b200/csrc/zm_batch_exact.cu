@@ -169,11 +169,12 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_exact_kernel(const Bat
         if (st > 0 && !grid_barrier(bp.bar, gridDim.x + bp.missing, bp.abort, bp.err, &s_ok)) return;
         const int op = bp.step[st].op;
         const BatchStep &S = bp.step[st];
-        int64_t tile = blockIdx.x;
-        int fi = tile < bp.tiles ? __ldg(bp.tile_field + tile) : 0;
-        for (; tile < bp.tiles; tile += gridDim.x) {
+        const int ntiles = (int)bp.tiles, hop = walks_back(bp, st) ? -(int)gridDim.x : (int)gridDim.x;
+        int tile = hop < 0 ? ntiles - 1 - (int)blockIdx.x : (int)blockIdx.x;
+        int fi = tile < ntiles ? __ldg(bp.tile_field + tile) : 0;
+        for (; (unsigned)tile < (unsigned)ntiles; tile += hop) {
             const BatchField &f = bp.fields[fi];
-            if (tile + gridDim.x < bp.tiles) fi = __ldg(bp.tile_field + tile + gridDim.x);
+            if ((unsigned)(tile + hop) < (unsigned)ntiles) fi = __ldg(bp.tile_field + tile + hop);
             const Geom &g = f.g;
             const int64_t sub = tile - f.tile0;   // of the field
             const cpx<float> *in = reinterpret_cast<const cpx<float> *>(S.in) + f.off;
