@@ -853,9 +853,8 @@ __global__ void __launch_bounds__(256) stencil3d_march_kernel(const cpx<S> *__re
         for (int k = waited; k < issued; k++) wait_bounded(k);
 }
 
-// The plane-tile 3D Laplacian where its shape applies (complex fields; tiles of
-// TY = min(8 complex64 / 4 complex128, B) rows dividing B and L; the four slots within
-// 200 KB of shared memory); cudaErrorNotSupported otherwise, and the caller uses
+// The plane-tile 3D Laplacian on tiles of TY rows (TY divides B and L), where its four slots
+// fit 200 KB of shared memory; cudaErrorNotSupported otherwise, and the caller uses
 // stencil3d_lines_kernel.
 template <typename S, int TY>
 static cudaError_t launch_march_ty(const zm_plan_s *p, const S *in, S *out, S coef, cudaStream_t st) {
@@ -894,15 +893,29 @@ static cudaError_t launch_march_ty(const zm_plan_s *p, const S *in, S *out, S co
                              reinterpret_cast<const cpx<S> *>(in), reinterpret_cast<cpx<S> *>(out), g, zsteps, coef,
                              p->dev_err);
 }
+// The plane-marching kernel, where it is the faster one; elsewhere the lines kernel, which gives
+// the same bits.  A march is one long walk per CTA over TY rows and their two halo rows, so it
+// needs a field that fills the chip (from N = 256: N = 128, P = 2, B = 8 22 us against 15 c64, 27
+// against 20 c128; N = 64 18 against 5) and a tall tile.  us, march / lines:
+//   * complex64, TY = 8 (B >= 8): N = 512, P = 4 518 / 671, P = 8 655 / 822, N = 256, P = 2
+//     70 / 84.  One rank per column (P = 1) only with vectors of at most 16: N = 512,
+//     B = 8 (vectors of 64) 665 / 512, N = 256, B = 8 (32) 79 / 71.  TY = 4 (B = 4): on rows of
+//     256 elements and up N = 512, P = 2 619 / 671; on shorter ones P = 4 781 / 712, N = 256,
+//     P = 4 153 / 108.  B = 2: N = 512, P = 4 1290 / 782, N = 256, P = 4 274 / 109.
+//   * complex128, TY = 4: vectors of at most 16, rows of 64 and up: N = 512, P = 4, B = 16
+//     886 / 1067, P = 8, B = 4 1271 / 1361, N = 256, P = 2, B = 16 117 / 141; longer vectors N = 512,
+//     P = 4, B = 4 1149 / 945, P = 2, B = 4 1592 / 908; shorter rows N = 256, P = 8, B = 4
+//     249 / 182.  B = 2: N = 512, P = 2 1497 / 899.
 template <typename S>
 static cudaError_t launch_march(const zm_plan_s *p, const S *in, S *out, S coef, cudaStream_t st) {
     const Geom &g = p->g;
-    const int64_t tymax = sizeof(S) == 4 ? 8 : 4;
-    const int64_t ty = g.b < tymax ? g.b : tymax;
-    if (g.dim != 3 || g.L % ty || g.b % ty || g.n < 16) return cudaErrorNotSupported;
-    if (ty == 8) return launch_march_ty<S, 8>(p, in, out, coef, st);
-    if (ty == 4) return launch_march_ty<S, 4>(p, in, out, coef, st);
-    if (ty == 2) return launch_march_ty<S, 2>(p, in, out, coef, st);
+    if (g.dim != 3 || g.n < 256) return cudaErrorNotSupported;
+    if constexpr (sizeof(S) == 4) {
+        if (g.b >= 8 && (g.p > 1 || g.vec <= 16)) return launch_march_ty<S, 8>(p, in, out, coef, st);
+        if (g.b == 4 && g.p > 1 && g.L >= 256) return launch_march_ty<S, 4>(p, in, out, coef, st);
+    } else {
+        if (g.b >= 4 && g.vec <= 16 && g.L >= 64) return launch_march_ty<S, 4>(p, in, out, coef, st);
+    }
     return cudaErrorNotSupported;
 }
 
