@@ -1,4 +1,6 @@
-// zm_fft2.cuh -- size-specialised fused axis pass (the fast path of zm_fft.cu).
+// zm_fft2.cuh -- fused axis pass specialised for VEC and M: complex128 lines of 2^14 points
+// (VEC = 64) and the variants that the tile-shape autotuner measures; every other size
+// defaults to the pass sized by N alone (zm_axis.cuh).
 //
 // Same computation as line_fft_kernel (see zm_fft.cu for how one pass replaces the
 // reference's FFT1a / pack / All-to-All / unpack+twiddle / FFT1b / repack stages), with
