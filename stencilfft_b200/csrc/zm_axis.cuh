@@ -98,8 +98,8 @@ template <typename T, int LN, int LTL, int LP, int LE> struct AxisCfg {
         return c;
     }
     // The persistent form is for tiles that leave room for one CTA per SM, where nothing else
-    // covers a tile's loads: N = 8192 c64 701 / 728 -> 664 / 669 us forward / inverse, c128
-    // 1402 / 1535 -> 1198 / 1393 (twiddles in tensor memory alone 695 / 730 and 1354 / 1479).
+    // covers a tile's loads: N = 8192 c64 701 / 728 -> 646 / 682 us forward / inverse, c128
+    // 1402 / 1535 -> 1182 / 1491 (twiddles in tensor memory alone 695 / 730 and 1354 / 1479).
     // With two CTAs or more it is no faster (N = 4096 c64 136 / 160 against 142 / 159, 3D
     // N = 256 c64 156 / 159 against 175 / 177), nor on one-line complex64 tiles of 2^14
     // points, whose strided side moves single elements (4266 / 3520 against 4472 / 4342).
@@ -108,8 +108,8 @@ template <typename T, int LN, int LTL, int LP, int LE> struct AxisCfg {
 
 // The weight tables as the kernel sees them: launch parameters, or a table in global memory
 // (batches, one per field layout).
-struct AxisParamMap {
-    static constexpr bool CONST_IN = true;    // the input is constant while the kernel runs
+template <bool CONST> struct AxisParamMapOf {
+    static constexpr bool CONST_IN = CONST;   // ld_field: a plain launch that does not write its input
     static constexpr int COMP64 = 2;          // compensated codelet constants in complex64 (dft)
     const AxisMap &m;
     ZM_DEV int va(int i) const { return m.va[i]; }
@@ -118,8 +118,9 @@ struct AxisParamMap {
     ZM_DEV int fs(int i) const { return m.fs[i]; }
     ZM_DEV int fr(int i) const { return m.fr[i]; }
 };
+using AxisParamMap = AxisParamMapOf<false>;
 struct AxisGlobalMap {
-    static constexpr bool CONST_IN = false;   // an earlier step of the launch may have written it
+    static constexpr bool CONST_IN = false;   // an earlier step of the launch wrote it
     static constexpr int COMP64 = 3;          // phi of 256 x 256^2: 1.86e-7 of FP64 with 2, 1.76e-7 with 3, 0.5 % slower
     const AxisMap *m;
     ZM_DEV int va(int i) const { return __ldg(m->va + i); }
@@ -164,13 +165,13 @@ struct AxisPass {
 #pragma unroll
             for (int r = 0; r < EPT; r += 2) {
                 const float4 *g = reinterpret_cast<const float4 *>(in + ra(r));
-                const float4 q = MAP::CONST_IN ? __ldg(g) : *g;
+                const float4 q = ld_field<MAP::CONST_IN>(g);
                 v[r] = {q.x, q.y};
                 v[r + 1] = {q.z, q.w};
             }
         } else {
 #pragma unroll
-            for (int r = 0; r < EPT; r++) v[r] = MAP::CONST_IN ? ldg(in + ra(r)) : in[ra(r)];
+            for (int r = 0; r < EPT; r++) v[r] = ld_field<MAP::CONST_IN>(in + ra(r));
         }
         if constexpr (BAR) __syncthreads();
 #pragma unroll
@@ -229,7 +230,7 @@ struct AxisPass {
             C *g = gm + axis_bits<LU>(u, [&](int b) { return m.fa(LNT + b); });
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                if constexpr (INV) x[r] = MAP::CONST_IN ? ldg(g + ga(r)) : g[ga(r)];
+                if constexpr (INV) x[r] = ld_field<MAP::CONST_IN>(g + ga(r));
                 else x[r] = s[axis_slot(r << LTL)];
             }
             dft<R, DIR, T, COMP>(x);
@@ -380,11 +381,12 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
 
 // The persistent form, one CTA per SM: CTA c walks tiles c, c + CTAs, ..., each thread's stage
 // twiddles (the same for every tile) in tensor memory, and asks for its next tile in L2 as
-// soon as it holds the current one.
-template <typename T, int LN, int LTL, int LP, int LE, bool INV>
+// soon as it holds the current one.  CONST: non-coherent loads, for inverse passes that do
+// not run in place, launched plainly (launch_axis).
+template <typename T, int LN, int LTL, int LP, int LE, bool INV, bool CONST>
 __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T, LN, LTL, LP, LE>::MINB))
     axis_tm_kernel(const __grid_constant__ AxisParams p, unsigned tiles) {
-    using A = AxisPass<T, LN, LTL, LP, LE, INV>;
+    using A = AxisPass<T, LN, LTL, LP, LE, INV, AxisParamMapOf<CONST>>;
     using CF = typename A::CF;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_tm;
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__((AxisCfg<T, LN, LTL, LP, LE>::NT), (AxisCfg<T,
     overlap_wait();
     const cpx<T> *in = reinterpret_cast<const cpx<T> *>(p.in);
     cpx<T> *out = reinterpret_cast<cpx<T> *>(p.out);
-    const AxisParamMap m{p.m};
+    const AxisParamMapOf<CONST> m{p.m};
 #pragma unroll 1
     for (unsigned c = blockIdx.x; c < tiles; c += gridDim.x) {
         const LineAddr la = line_addr(p.g, p.kind, (int64_t)c << LTL, p.m.lg);
@@ -438,11 +440,18 @@ cudaError_t launch_axis(const AxisParams &p, int64_t nlines, cudaStream_t st) {
         static int resident[64] = {0};
         int dev = 0;
         cudaGetDevice(&dev);
-        auto ktm = axis_tm_kernel<T, LN, LTL, LP, LE, INV>;
+        // The inverse's strided loads are faster non-coherent (N = 8192, us per transform, coherent /
+        // non-coherent: c64 704 / 682, c128 1545 / 1491; the forward's are not, c64 645 / 673), which
+        // is right only for an input that nothing writes while the kernel runs: not in place, and
+        // launched plainly, after all that came before it.
+        auto ktm = axis_tm_kernel<T, LN, LTL, LP, LE, INV, false>;
+        auto kconst = axis_tm_kernel<T, LN, LTL, LP, LE, INV, INV>;
         int ctas = dev < 64 ? resident[dev] : 0;
         if (!ctas) {
             int sms = 0;
             cudaError_t e = cudaFuncSetAttribute(ktm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
+            if (e == cudaSuccess && INV)
+                e = cudaFuncSetAttribute(kconst, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return e;
             ctas = sms;   // one per SM
@@ -450,6 +459,10 @@ cudaError_t launch_axis(const AxisParams &p, int64_t nlines, cudaStream_t st) {
         }
         if (tiles >= 3 * (unsigned)ctas) {
             count_launch();
+            if (INV && p.in != p.out) {
+                kconst<<<(unsigned)ctas, CF::NT, CF::SMEM, st>>>(p, tiles);
+                return cudaGetLastError();
+            }
             return launch_overlapped(ktm, (unsigned)ctas, CF::NT, CF::SMEM, st, p, tiles);
         }
     }

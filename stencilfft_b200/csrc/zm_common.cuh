@@ -100,14 +100,44 @@ template <> ZM_DEV tw<float> ldtw(const tw<float> *t, int64_t i) {
     return {v.x, v.y, v.z, v.w};
 }
 
-template <typename R> ZM_DEV cpx<R> ldg(const cpx<R> *p) { return *p; }
-template <> ZM_DEV cpx<double> ldg(const cpx<double> *p) {
-    double2 v = __ldg(reinterpret_cast<const double2 *>(p));
-    return {v.x, v.y};
-}
-template <> ZM_DEV cpx<float> ldg(const cpx<float> *p) {
-    float2 v = __ldg(reinterpret_cast<const float2 *>(p));
-    return {v.x, v.y};
+// A load of field data.  __ldg is for tables that were uploaded when the plan was made: a
+// field is in general not constant while a kernel runs.  An overlapped launch begins while
+// the kernel before it still writes, y passes run in place, and a batch step reads what the
+// step before it wrote; a non-coherent load may then return what the SM read before that
+// write, and the compiler may move it above the wait.  So fields are read by coherent loads,
+// here in the order of the source and behind overlap_wait; a plain dereference is as good
+// where the compiler's own order is faster, of a pointer without __restrict__ (which would
+// make it a non-coherent load).  CONST: a non-coherent load, for a kernel that is launched
+// plainly and does not write its input.
+template <bool CONST = false, typename V> ZM_DEV V ld_field(const V *p) {
+    static_assert(sizeof(V) == 4 || sizeof(V) == 8 || sizeof(V) == 16, "4, 8 or 16 bytes");
+    const unsigned long long a = (unsigned long long)__cvta_generic_to_global(p);
+    V v;
+    if constexpr (sizeof(V) == 16) {
+        if constexpr (CONST) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+            memcpy(&v, &q, 16);
+        } else {
+            unsigned long long q[2];
+            asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(q[0]), "=l"(q[1]) : "l"(a) : "memory");
+            memcpy(&v, q, 16);
+        }
+    } else if constexpr (sizeof(V) == 8) {
+        if constexpr (CONST) {
+            const float2 q = __ldg(reinterpret_cast<const float2 *>(p));
+            memcpy(&v, &q, 8);
+        } else {
+            unsigned long long q;
+            asm volatile("ld.global.b64 %0, [%1];" : "=l"(q) : "l"(a) : "memory");
+            memcpy(&v, &q, 8);
+        }
+    } else {
+        static_assert(!CONST, "no caller");
+        unsigned q;
+        asm volatile("ld.global.b32 %0, [%1];" : "=r"(q) : "l"(a) : "memory");
+        memcpy(&v, &q, 4);
+    }
+    return v;
 }
 
 // ------------------------------------------- per-thread asynchronous copies (cp.async)
@@ -128,7 +158,7 @@ ZM_DEV void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "mem
 // ------------------------------------------------ overlapped launches (launch_overlapped)
 // Let the next kernel of the stream be scheduled as this one's CTAs leave; wait until every
 // earlier kernel has finished and its writes are visible.  Every thread waits before its
-// first access to a field, so a kernel only ever overlaps another's scheduling and index
+// first access to a field and reads fields by coherent loads (ld_field), so a kernel only ever overlaps another's scheduling and index
 // arithmetic.  Only the axis passes let the next kernel in early: from the 3D Laplacian, whose
 // CTAs walk long columns, its waiting CTAs took resources (3D N = 512 c64 round trip +
 // Laplacian 3.00 -> 3.58 ms); the other kernels only wait.

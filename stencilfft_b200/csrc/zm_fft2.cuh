@@ -42,7 +42,7 @@
 namespace zm {
 
 template <typename T> ZM_DEV uint4 ldg16(const cpx<T> *p) {
-    return __ldg(reinterpret_cast<const uint4 *>(p));
+    return ld_field(reinterpret_cast<const uint4 *>(p));
 }
 
 template <int CL> ZM_DEV void tile_sync() {
@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(NT, (fused_min_blocks<T, LV, LM, CL, TL, NT, I
                 for (int i = 0; i < NU; i++) {
                     const C *row = in + arow(ut[i], un1[i]) + uj[i] * apos;
 #pragma unroll
-                    for (int r = 0; r < RA1; r++) v[i][r] = ldg(row + RA2 * r * apos);
+                    for (int r = 0; r < RA1; r++) v[i][r] = ld_field(row + RA2 * r * apos);
                 }
             }
 #pragma unroll
@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(NT, (fused_min_blocks<T, LV, LM, CL, TL, NT, I
                     for (int i = 0; i < NU; i++) {
                         const uint4 *rp = reinterpret_cast<const uint4 *>(in + arow(ut[i], un1[i]));
 #pragma unroll
-                        for (int q = 0; q < RA1 * (int)sizeof(C) / 16; q++) buf[i][q] = __ldg(rp + q);
+                        for (int q = 0; q < RA1 * (int)sizeof(C) / 16; q++) buf[i][q] = ld_field(rp + q);
                     }
 #pragma unroll
                     for (int i = 0; i < NU; i++) memcpy(&v[i][0], &buf[i][0], RA1 * sizeof(C));
@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(NT, (fused_min_blocks<T, LV, LM, CL, TL, NT, I
                 for (int i = 0; i < NU; i++) {
                     const C *ip = fptr(in, zt[i], k2_0 + zk[i], zj[i]);
 #pragma unroll
-                    for (int r = 0; r < RC1; r++) z[i][r] = ldg(ip + fstep1() * r);
+                    for (int r = 0; r < RC1; r++) z[i][r] = ld_field(ip + fstep1() * r);
                 }
             }
 #pragma unroll

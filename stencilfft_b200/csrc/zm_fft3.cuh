@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(512, 1) k3_pass_kernel(const LineParams prm) {
                 if constexpr (vcont) {
 #pragma unroll
                     for (int d2 = 0; d2 < 16; d2++) {
-                        const float4 v = __ldg(reinterpret_cast<const float4 *>(row + voff(lo0 + DSTEP * d2)));
+                        const float4 v = ld_field(reinterpret_cast<const float4 *>(row + voff(lo0 + DSTEP * d2)));
                         x0[d2] = C{v.x, v.y};
                         x1[d2] = C{v.z, v.w};
                     }
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(512, 1) k3_pass_kernel(const LineParams prm) {
                     float4 v[16];
 #pragma unroll
                     for (int d2 = 0; d2 < 16; d2++)
-                        v[d2] = __ldg(reinterpret_cast<const float4 *>(prow + voff(lob + DSTEP * d2)));
+                        v[d2] = *reinterpret_cast<const float4 *>(prow + voff(lob + DSTEP * d2));
                     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // partner running
 #pragma unroll
                     for (int d2 = 0; d2 < 16; d2++) {
@@ -286,8 +286,8 @@ __global__ void __launch_bounds__(512, 1) k3_pass_kernel(const LineParams prm) {
                 } else {
 #pragma unroll
                     for (int d2 = 0; d2 < 16; d2++) {
-                        x0[d2] = ldg(row + voff(lo0 + DSTEP * d2));
-                        x1[d2] = ldg(row + voff(lo1 + DSTEP * d2));
+                        x0[d2] = ld_field(row + voff(lo0 + DSTEP * d2));
+                        x1[d2] = ld_field(row + voff(lo1 + DSTEP * d2));
                     }
                 }
             }
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(512, 1) k3_pass_kernel(const LineParams prm) {
             } else {
                 const C *ip = in + fofs(a);
 #pragma unroll
-                for (int kc = 0; kc < 32; kc++) y[kc] = ldg(ip + fstep * kc);
+                for (int kc = 0; kc < 32; kc++) y[kc] = ld_field(ip + fstep * kc);
             }
             dft<32, DIR, float>(y);
             __syncthreads();   // tables written; staging fully read

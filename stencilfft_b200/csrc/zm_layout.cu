@@ -33,7 +33,7 @@ __host__ __device__ constexpr int perm_slot(int i) { return i + (i >> 4) + (i >>
 
 // E = 2^LE elements per tile, 2^(LE - 8) per thread
 template <typename T, int LE>
-__global__ void __launch_bounds__(256) permute_kernel(const cpx<T> *__restrict__ in, cpx<T> *__restrict__ out,
+__global__ void __launch_bounds__(256) permute_kernel(const cpx<T> *in, cpx<T> *out,
                                                       const __grid_constant__ PermMap m) {
     constexpr int LP = LE > 8 ? LE - 8 : 0, LNT = LE - LP, EPT = 1 << LP;
     constexpr bool PAIR = sizeof(T) == 4 && LP >= 1;   // 16-byte accesses: address bit 0 in the registers
@@ -75,11 +75,11 @@ __global__ void __launch_bounds__(256) permute_kernel(const cpx<T> *__restrict__
 #pragma unroll
     for (int r = 0; r < EPT; r += 1 + R0) {
         if constexpr (PAIR) {
-            const float4 q = __ldg(reinterpret_cast<const float4 *>(in + bi + off(r, m.ia)));
+            const float4 q = ld_field(reinterpret_cast<const float4 *>(in + bi + off(r, m.ia)));
             v[r] = {q.x, q.y};
             v[r + 1] = {q.z, q.w};
         } else {
-            v[r] = ldg(in + bi + off(r, m.ia));
+            v[r] = ld_field(in + bi + off(r, m.ia));
         }
     }
 #pragma unroll
@@ -210,7 +210,7 @@ template <typename T> ZM_DEV void ld_run(const cpx<T> *p, cpx<T> *v) {
     constexpr int NV = CEPT * (int)sizeof(cpx<T>) / 16;
 #pragma unroll
     for (int q = 0; q < NV; q++)
-        reinterpret_cast<uint4 *>(v)[q] = __ldg(reinterpret_cast<const uint4 *>(p) + q);
+        reinterpret_cast<uint4 *>(v)[q] = ld_field(reinterpret_cast<const uint4 *>(p) + q);
 }
 template <typename T> ZM_DEV void st_run(cpx<T> *p, const cpx<T> *v) {
     constexpr int NV = CEPT * (int)sizeof(cpx<T>) / 16;
@@ -228,7 +228,7 @@ template <typename T> ZM_DEV void st_run(cpx<T> *p, const cpx<T> *v) {
 // per bit, so layouts with VP < 4 take no full map per element either (N = 4096 c64,
 // VP = 1: 92 -> 43 us, VP >= 4: 43 / 45 -> 43; c128 107 -> 93 / 104 us; Gaussian / Poisson).
 template <typename T, typename I>
-__global__ void __launch_bounds__(256) spectral_kernel(cpx<T> *__restrict__ d, const Geom g, int64_t total, int op,
+__global__ void __launch_bounds__(256) spectral_kernel(cpx<T> *d, const Geom g, int64_t total, int op,
                                                        double a) {
     const int64_t e0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * CEPT;
     overlap_wait();

@@ -80,9 +80,8 @@ template <> ZM_DEV double div_den<double>(double x, double den, double) { return
 template <> ZM_DEV float div_den<float>(float x, float, float rden) { return __fmul_rn(x, rden); }
 
 template <typename S, int NC, int OP, int DIM>
-__global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, S *__restrict__ out,
-                                                      S *__restrict__ out2, S *__restrict__ out3,
-                                                      const Geom g, int64_t nvec, S coef, S coef2, S rden) {
+__global__ void __launch_bounds__(256) stencil_kernel(const S *in, S *out, S *out2, S *out3, const Geom g,
+                                                      int64_t nvec, S coef, S coef2, S rden) {
     using O = ops<S>;
     using V = vec16<S>;
     constexpr int K = V::n / NC;                 // elements per vector
@@ -117,12 +116,12 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
     auto vrow = [&](int d) {
         int id, li;
         g2l((gr + d + N) & (N - 1), g, id, li);
-        return __ldg(reinterpret_cast<const uint4 *>(in + addr(rank_of(did, id, cid), ld, li, pos) * NC));
+        return *reinterpret_cast<const uint4 *>(in + addr(rank_of(did, id, cid), ld, li, pos) * NC);
     };
     auto vdep = [&](int d) {
         int id, li;
         g2l((gd + d + N) & (N - 1), g, id, li);
-        return __ldg(reinterpret_cast<const uint4 *>(in + addr(rank_of(id, rid, cid), li, lr, pos) * NC));
+        return *reinterpret_cast<const uint4 *>(in + addr(rank_of(id, rid, cid), li, lr, pos) * NC);
     };
     // neighbour along x (columns) at column offset d of the K elements
     auto vcol = [&](int d) {
@@ -130,8 +129,8 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
         const int j = pos >> g.logVEC;
         if (j + d >= 0 && j + d < (int)g.b && (K == 1 || (int)g.vec % K == 0)) {
             // same rank and same jj: the neighbour vector is d packed vectors away
-            *reinterpret_cast<uint4 *>(&r) = __ldg(reinterpret_cast<const uint4 *>(
-                in + (e + (int64_t)d * (int64_t)g.vec) * NC));
+            *reinterpret_cast<uint4 *>(&r) = *reinterpret_cast<const uint4 *>(
+                in + (e + (int64_t)d * (int64_t)g.vec) * NC);
             return r;
         }
         const int gc0 = pos2gc(pos, cid, g);
@@ -148,7 +147,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
             contiguous = idl == id0 && pl == p0 + K - 1 && (p0 & (K - 1)) == 0;
         }
         if (contiguous) {
-            *reinterpret_cast<uint4 *>(&r) = __ldg(reinterpret_cast<const uint4 *>(in + a0 * NC));
+            *reinterpret_cast<uint4 *>(&r) = *reinterpret_cast<const uint4 *>(in + a0 * NC);
         } else {
 #pragma unroll
             for (int k = 0; k < K; k++) {
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
                 gc2pos((pos2gc(pos + k, cid, g) + d + N) & (N - 1), g, idk, pk);
                 const int64_t ak = addr(rank_of(did, rid, idk), ld, lr, pk);
 #pragma unroll
-                for (int q = 0; q < NC; q++) r.v[k * NC + q] = __ldg(in + ak * NC + q);
+                for (int q = 0; q < NC; q++) r.v[k * NC + q] = in[ak * NC + q];
             }
         }
         return r;
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
     if (OP == ST_ALL) {
         const V up = as(vrow(-1)), dn = as(vrow(1)), lf = vcol(-1), rt = vcol(1);
         const V up2 = as(vrow(-2)), dn2 = as(vrow(2)), lf2 = vcol(-2), rt2 = vcol(2);
-        const V c = as(__ldg(reinterpret_cast<const uint4 *>(in + e * NC)));
+        const V c = as(*reinterpret_cast<const uint4 *>(in + e * NC));
         V rx, ry;
         const S den = O::mul((S)12, coef2);
 #pragma unroll
@@ -197,7 +196,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
     } else if (OP == ST_LAPLACE) {
         // laplace.cu:91-168 / laplace3d.cu:98-224 accumulation order
         const V up = as(vrow(-1)), dn = as(vrow(1)), lf = vcol(-1), rt = vcol(1);
-        const V c = as(__ldg(reinterpret_cast<const uint4 *>(in + e * NC)));
+        const V c = as(*reinterpret_cast<const uint4 *>(in + e * NC));
         V fr, bk;
         if (DIM == 3) {
             fr = as(vdep(-1));
@@ -244,9 +243,9 @@ __global__ void __launch_bounds__(256) stencil_kernel(const S *__restrict__ in, 
 // outputs, and the index arithmetic is done once per thread.  Rows outside the block
 // (above a block's first row group, below its last) go through the block-cyclic maps as
 // in stencil_kernel; every output is computed by the same expressions, in the same order.
-template <typename S, int NC, int OP, int RY>
-ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *__restrict__ out2,
-                              S *__restrict__ out3, const Geom &g, int64_t nthreads, S coef, S coef2, S rden) {
+template <typename S, int NC, int OP, int RY, bool CONST = false>
+ZM_DEV void stencil_rows_body(const S *in, S *out, S *out2, S *out3, const Geom &g, int64_t nthreads, S coef,
+                              S coef2, S rden) {
     using O = ops<S>;
     using V = vec16<S>;
     constexpr int K = V::n / NC;                 // elements per vector
@@ -268,7 +267,7 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
     const int lrb0 = lr0 & ((int)g.b - 1);
     auto ld16 = [&](int64_t el) {
         V r;
-        *reinterpret_cast<uint4 *>(&r) = __ldg(reinterpret_cast<const uint4 *>(in + el * NC));
+        *reinterpret_cast<uint4 *>(&r) = ld_field<CONST>(reinterpret_cast<const uint4 *>(in + el * NC));
         return r;
     };
     // row lr0 + d (d in [-2, RY + 1]) at the same packed position
@@ -302,7 +301,7 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
             gc2pos((pos2gc(pos + k, cid, g) + d + N) & (N - 1), g, idk, pk);
             const int64_t ak = ((int64_t)(rid * P + idk) << (2 * g.logL)) + (int64_t)lr * L + pk;
 #pragma unroll
-            for (int q = 0; q < NC; q++) r.v[k * NC + q] = __ldg(in + ak * NC + q);
+            for (int q = 0; q < NC; q++) r.v[k * NC + q] = ld_field<CONST>(in + ak * NC + q);
         }
         return r;
     };
@@ -456,18 +455,21 @@ ZM_DEV void stencil_rows_body(const S *__restrict__ in, S *__restrict__ out, S *
 // in place of the FP64 division was slower (dx 113 -> 121 us at N = 4096: the division's own
 // fast path is as short as the range checks that this takes).
 template <typename S, int NC, int OP, int RY>
-__global__ void __launch_bounds__(256) stencil_rows_kernel(const S *__restrict__ in, S *__restrict__ out,
-                                                           S *__restrict__ out2, S *__restrict__ out3,
-                                                           const Geom g, int64_t nthreads, S coef, S coef2,
-                                                           S rden) {
+__global__ void __launch_bounds__(256) stencil_rows_kernel(const S *in, S *out, S *out2, S *out3, const Geom g,
+                                                           int64_t nthreads, S coef, S coef2, S rden) {
     stencil_rows_body<S, NC, OP, RY>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
 }
 template <typename S, int NC, int OP, int RY, int MB>
-__global__ void __launch_bounds__(256, MB) stencil_rowsb_kernel(const S *__restrict__ in, S *__restrict__ out,
-                                                               S *__restrict__ out2, S *__restrict__ out3,
-                                                               const Geom g, int64_t nthreads, S coef, S coef2,
-                                                               S rden) {
+__global__ void __launch_bounds__(256, MB) stencil_rowsb_kernel(const S *in, S *out, S *out2, S *out3, const Geom g,
+                                                                int64_t nthreads, S coef, S coef2, S rden) {
     stencil_rows_body<S, NC, OP, RY>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
+}
+// Plainly launched, with non-coherent loads: the three FP64 stencils of a large field in one
+// launch (launch_s).
+template <typename S, int NC, int OP, int RY, int MB>
+__global__ void __launch_bounds__(256, MB) stencil_rowsc_kernel(const S *in, S *out, S *out2, S *out3, const Geom g,
+                                                                int64_t nthreads, S coef, S coef2, S rden) {
+    stencil_rows_body<S, NC, OP, RY, true>(in, out, out2, out3, g, nthreads, coef, coef2, rden);
 }
 
 // 3D Laplacian (laplace3d.cu:98-224 accumulation order) with RX vectors of one line per
@@ -479,8 +481,7 @@ __global__ void __launch_bounds__(256, MB) stencil_rowsb_kernel(const S *__restr
 // (stencil_kernel<..., 3>).  Each output is computed by the same expressions in the same
 // order as there.
 template <typename S, int NC, int RX>
-__global__ void __launch_bounds__(256) stencil3d_lines_kernel(const S *__restrict__ in, S *__restrict__ out,
-                                                              const Geom g, int64_t nseg, S coef) {
+__global__ void __launch_bounds__(256) stencil3d_lines_kernel(const S *in, S *out, const Geom g, int64_t nseg, S coef) {
     overlap_wait();
     using O = ops<S>;
     using V = vec16<S>;
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(256) stencil3d_lines_kernel(const S *__restric
     const int64_t ec = line << g.logL, eu = yline(-1), ed = yline(1), ef = zline(-1), eb = zline(1);
     auto ld16 = [&](int64_t el) {
         V r;
-        *reinterpret_cast<uint4 *>(&r) = __ldg(reinterpret_cast<const uint4 *>(in + el * NC));
+        *reinterpret_cast<uint4 *>(&r) = *reinterpret_cast<const uint4 *>(in + el * NC);
         return r;
     };
     // neighbour along x (d = -1 / +1) of the vector at packed position pos (VEC a multiple
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(256) stencil3d_lines_kernel(const S *__restric
         for (int k = 0; k < K; k++) {
             const int64_t ak = e1 + ((jj + k + d) & ((int)g.vec - 1));
 #pragma unroll
-            for (int q = 0; q < NC; q++) r.v[k * NC + q] = __ldg(in + ak * NC + q);
+            for (int q = 0; q < NC; q++) r.v[k * NC + q] = in[ak * NC + q];
         }
         return r;
     };
@@ -646,7 +647,7 @@ template <int N> ZM_DEV void st_cp_wait() { asm volatile("cp.async.wait_group %0
 // bounded waits raises the plan's device error word; the CTA then stops, after its copies
 // in flight have landed (bounded).
 template <typename S, int TY>
-__global__ void __launch_bounds__(256) stencil3d_march_kernel(const cpx<S> *__restrict__ in, cpx<S> *__restrict__ out,
+__global__ void __launch_bounds__(256) stencil3d_march_kernel(const cpx<S> *in, cpx<S> *out,
                                                               const Geom g, int zsteps, S coef, int *err) {
     using C = cpx<S>;
     using O = ops<S>;
@@ -948,13 +949,21 @@ static cudaError_t launch_s(const zm_plan_s *p, int op, const void *in, void *ou
             // two, 86 / 45 with four).  Laplacian: two rows (109 -> 104; at B = 4, 129 -> 131,
             // one row stays better).  dx shares no rows (113 with one, 119 with two), and the
             // three in one launch hold too many registers with more than one (221 against 238).
+            // They are slower with coherent loads, whose order the compiler keeps: fields large
+            // enough to pay for a plain launch take non-coherent ones (N = 4096 239 -> 223, N = 2048
+            // 61.7 -> 59.5, but N = 1024 14.5 -> 16.5).
             if (op == ST_DY && p->g.b % 4 == 0) ZM_ROWSB(ST_DY, 4, 4);
             else if (op == ST_DY && p->g.b % 2 == 0) ZM_ROWSB(ST_DY, 2, 5);
             else if (op == ST_DY) ZM_ROWSB(ST_DY, 1, 5);
             else if (op == ST_LAPLACE && p->g.b % 8 == 0) ZM_ROWSB(ST_LAPLACE, 2, 5);
             else if (op == ST_LAPLACE) ZM_ROWSB(ST_LAPLACE, 1, 5);
             else if (op == ST_DX) ZM_ROWSB(ST_DX, 1, 5);
-            else ZM_ROWSB(ST_ALL, 1, 5);
+            else if (p->g.logN < 11) ZM_ROWSB(ST_ALL, 1, 5);
+            else {
+                stencil_rowsc_kernel<S, NC, ST_ALL, 1, 5><<<blocks(1), threads, 0, st>>>(i, o, o2, o3, p->g, nvec, c,
+                                                                                         c2, rd);
+                e = cudaGetLastError();
+            }
         } else if (p->g.b % 4 == 0) {
             // FP32: four rows of a B-row block per thread
             if (op == ST_LAPLACE) ZM_ROWS(ST_LAPLACE, 4);

@@ -298,7 +298,7 @@ ZM_DEV void tile_load_vec(const Tile &c, const Geom &g, cpx<T> *s, const cpx<T> 
         const int t = e >> g.logN;
         const int r = e & (int)(g.n - 1);
         const int ch = r >> g.logL, pos = r & (int)(g.L - 1);
-        v[i] = ldg(in + c.abase[t] + ch * c.a_chunk + pos);
+        v[i] = ld_field(in + c.abase[t] + ch * c.a_chunk + pos);
     }
 #pragma unroll
     for (int i = 0; i < EPT; i++) s[SW::f(tid + i * nthr)] = v[i];
@@ -312,7 +312,7 @@ ZM_DEV void tile_load_freq(const Tile &c, const Geom &g, cpx<T> *s, const cpx<T>
     for (int i = 0; i < EPT; i++) {
         int t, ch, pos;
         tile_freq_coords(c, g, tid + i * nthr, t, ch, pos);
-        v[i] = ldg(in + c.fbase[t] + ch * c.f_chunk + pos * c.f_pos);
+        v[i] = ld_field(in + c.fbase[t] + ch * c.f_chunk + pos * c.f_pos);
     }
 #pragma unroll
     for (int i = 0; i < EPT; i++) {
@@ -385,8 +385,8 @@ ZM_DEV void tile_load_rows_v4(const Tile &c, cpx<float> *s, const cpx<float> *in
         const int t = rho >> LM, r = (rho & (M - 1)) << 2;
         const int off = (int)c.abase[t] + (r >> G::LL) * G::CHUNK + (r & (G::L - 1));
         const float4 *p = reinterpret_cast<const float4 *>(in + off);
-        v[q][0] = __ldg(p);
-        v[q][1] = __ldg(p + 1);
+        v[q][0] = ld_field(p);
+        v[q][1] = ld_field(p + 1);
     }
 #pragma unroll
     for (int q = 0; q < RPT; q++) {
@@ -444,7 +444,7 @@ ZM_DEV void tile_freq_v4(const Tile &c, cpx<float> *s, const cpx<float> *in, cpx
         for (int i = 0; i < EPT; i++) {
             int slot, off;
             coords(i, slot, off);
-            v[i] = ldg(in + off);
+            v[i] = ld_field(in + off);
         }
 #pragma unroll
         for (int i = 0; i < EPT; i++) {
