@@ -149,7 +149,9 @@ int zm_autotune_b(int dim, int64_t n, int64_t p, int dtype, int reps, int64_t *b
  * device_buf0, output in device_buf1, buf0 clobbered; fft.cu:189-198) -- unless the
  * plan was created with ZM_FLAG_OWN_WORKSPACE, whose workspace is then used; or a
  * buffer of zm_plan_workspace_size bytes, in which case `in` is preserved.  The
- * 2D forward transform never touches `in`.  With ZM_FLAG_PERMUTE_ONLY the calls
+ * 2D forward transform never touches `in`.  A workspace that overlaps `in` or `out` is
+ * refused, except by the 2D forward transform of layouts that need none (all but
+ * N = 16384 at VEC = 64 and complex64 N = 8192 at VEC = 32 and 64), which leaves it alone.  With ZM_FLAG_PERMUTE_ONLY the calls
  * reproduce the reference's do_compute=false pipelines (pure data movement).
  */
 int zm_fft_forward(zm_plan plan, const void *in, void *out, void *work, void *stream);
