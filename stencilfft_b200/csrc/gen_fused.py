@@ -6,14 +6,19 @@ for complex64 lines of 2^14 points ("k3p": its persistent form with asynchronous
 of the next line; "k3c": the forward y pass on buddy-line CTA pairs); "t" marks the
 persistent form of the fused pass whose next tile's first-phase points are staged in
 tensor memory (one CTA per SM).  Variant 0, the default, is the axis pass of zm_axis.cuh
-(no instance here: zm_api.cu launches it) except for lines of 2^14 points at VEC = 64,
-M = 256, where it is the first entry of the list; the others are the
-alternatives that zm_plan_autotune measures for a plan."""
+(no instance here: zm_api.cu launches it) except where the axis pass has no tile, and it is
+the first entry of the list: lines of 2^14 points at VEC = 64, M = 256, and complex64 lines
+of 2^11 points, whose 3D field has more elements than the axis pass' 32-bit offsets
+(axis_tile, zm_axis.cu) reach.  The other entries are the alternatives that
+zm_plan_autotune measures for a plan."""
 
 
-def axis_default(lv, lm):
-    return (lv, lm) != (6, 8)
-
+def axis_default(dt, lv, lm):
+    """Whether the axis pass runs every field of these lines that a 180 GB GPU holds twice."""
+    if (lv, lm) == (6, 8):
+        return False
+    eb = 8 if dt == "c64" else 16
+    return not any(2 ** 31 <= 2 ** (dim * (lv + lm)) <= 180e9 / (2 * eb) for dim in (2, 3))
 
 
 VARIANTS = {
@@ -80,7 +85,7 @@ for dt, table in VARIANTS.items():
              "    switch ((prm.g.logVEC << 16) | (prm.g.logM << 8) | prm.variant) {"]
         for (lv, lm), vs in table.items():
             for vi, v in enumerate(vs):
-                if vi == 0 and axis_default(lv, lm):
+                if vi == 0 and axis_default(dt, lv, lm):
                     continue
                 cl, tl, nt = v[:3]
                 pers = "true" if len(v) > 3 and v[3] == "p" else "false"
@@ -108,7 +113,7 @@ for dt, table in VARIANTS.items():
                   "    switch ((logvec << 16) | (logm << 8) | variant) {"]
             for (lv, lm), vs in table.items():
                 for vi, v in enumerate(vs):
-                    if vi == 0 and axis_default(lv, lm):
+                    if vi == 0 and axis_default(dt, lv, lm):
                         continue
                     cl, tl, nt = v[:3]
                     vec, n = 1 << lv, 1 << (lv + lm)

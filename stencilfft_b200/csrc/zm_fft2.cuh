@@ -1,6 +1,7 @@
 // zm_fft2.cuh -- fused axis pass specialised for VEC and M: complex128 lines of 2^14 points
-// (VEC = 64) and the variants that the tile-shape autotuner measures; every other size
-// defaults to the pass sized by N alone (zm_axis.cuh).
+// (VEC = 64), 3D complex64 fields of N = 2048 (VEC = 32), and the variants that the
+// tile-shape autotuner measures; the other sizes default to the pass sized by N alone
+// (zm_axis.cuh), as far as its 32-bit offsets reach (fields below 2^31 elements).
 //
 // Same computation as line_fft_kernel (see zm_fft.cu for how one pass replaces the
 // reference's FFT1a / pack / All-to-All / unpack+twiddle / FFT1b / repack stages), with

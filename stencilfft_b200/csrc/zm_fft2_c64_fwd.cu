@@ -14,6 +14,7 @@ cudaError_t launch_fused_c64_fwd(const LineParams &prm, cudaStream_t st, bool *h
     case (2 << 16) | (7 << 8) | 1: return launch_fused<float, 2, 7, 1, 16, 512, false, false>(prm, st);
     case (2 << 16) | (7 << 8) | 2: return launch_fused<float, 2, 7, 1, 32, 1024, false, false>(prm, st);
     case (2 << 16) | (7 << 8) | 3: return launch_fused<float, 2, 7, 1, 4, 128, false, false>(prm, st);
+    case (5 << 16) | (6 << 8) | 0: return launch_fused<float, 5, 6, 1, 4, 512, false, false>(prm, st);
     case (5 << 16) | (7 << 8) | 1: return launch_fused<float, 5, 7, 2, 2, 256, false, false>(prm, st);
     case (5 << 16) | (7 << 8) | 2: return launch_fused<float, 5, 7, 2, 4, 512, false, false>(prm, st);
     case (5 << 16) | (7 << 8) | 3: return launch_fused<float, 5, 7, 1, 1, 256, false, false>(prm, st);
@@ -61,6 +62,7 @@ int fused_variants_c64(int logvec, int logm) {
 
 int fused_interleave_lg_c64(int logvec, int logm, int variant) {
     switch ((logvec << 16) | (logm << 8) | variant) {
+    case (5 << 16) | (6 << 8) | 0: return 2;
     case (5 << 16) | (7 << 8) | 1: return 1;
     case (5 << 16) | (7 << 8) | 2: return 2;
     case (5 << 16) | (7 << 8) | 4: return 2;
