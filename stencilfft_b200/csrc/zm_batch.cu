@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPara
             // element-wise steps over the pass steps' tiles: tile `tile` of field f covers
             // elements [(tile - tile0) * TP, + TP) of the field's array (N^2 / TP tiles of a
             // field of N^2 elements), so every CTA has work whatever the field sizes
-            constexpr int TP = kBatchThreads * EPT;
+            constexpr int TP0 = kBatchThreads * EPT;
             for (int64_t tile = blockIdx.x; tile < bp.tiles; tile += gridDim.x) {
                 __syncthreads();   // the previous tile is done with sf
                 if (tid == 0) {
@@ -187,6 +187,8 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPara
                 __syncthreads();
                 const int f = s_f;
                 const Geom g = sf.g;
+                const bool half = g.n * g.n < TP0;   // a field smaller than a tile is a tile of its own
+                const int TP = half ? TP0 / 2 : TP0;
                 const int64_t e0 = (tile - sf.tile0) * TP;
                 cpx<T> *out = reinterpret_cast<cpx<T> *>(S.out) + sf.off;
                 if (S.op == BOP_FILL) {
@@ -208,12 +210,14 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPara
                 }
                 const cpx<T> *in = reinterpret_cast<const cpx<T> *>(S.in) + sf.off;
                 const cpx<T> *rhs = reinterpret_cast<const cpx<T> *>(S.aux) + sf.off;
-                residual_tile<T, TP>(g, S.a, in, rhs, out, e0, s, tid);
+                if (half) residual_tile<T, TP0 / 2>(g, S.a, in, rhs, out, e0, s, tid);
+                else residual_tile<T, TP0>(g, S.a, in, rhs, out, e0, s, tid);
             }
             continue;
         }
 
-        // axis-pass steps: tiles of TL lines, TL * N = nthr * EPT points
+        // axis-pass steps: tiles of TL lines, TL * N = nthr * EPT points (complex128 N = 32: the
+        // field's 32 lines, half as many)
         for (int64_t tile = blockIdx.x; tile < bp.tiles; tile += gridDim.x) {
             __syncthreads();   // the previous tile is done with sf, the bases and s
             if (tid == 0) sf = bp.fields[field_of_tile(bp.fields, bp.nfields, tile)];
@@ -246,6 +250,12 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(const BatchPara
                 }
             }
 #undef ZM_BT
+            if constexpr (sizeof(T) == 8) {
+                if (g.n * g.n < kBatchThreads * EPT) {
+                    done = true;
+                    batch_tile<T, EPT / 2, 0, SwzNone>(S.op, S.scale != 0, S.a, sf, c, s, in, out, l0, nthr, tid);
+                }
+            }
             if (!done) batch_tile<T, EPT, 0, SwzNone>(S.op, S.scale != 0, S.a, sf, c, s, in, out, l0, nthr, tid);
         }
     }
@@ -564,9 +574,10 @@ int zm_batch_create(zm_batch *batch, int nfields, const int64_t *n, const int64_
         f.off = B->elems;
         f.tile0 = B->tiles;
         f.twN = pl->twN;
-        f.T = (int)(tile_pts / n[i]);
-        f.nst_vec = zm::radix_schedule(pl->g.vec, ept, f.rad_vec);
-        f.nst_m = zm::radix_schedule(pl->g.m, ept, f.rad_m);
+        f.T = (int)std::min(tile_pts / n[i], n[i]);   // complex128 N = 32 has half a tile's points
+        const int fept = (int)(f.T * n[i] / zm::kBatchThreads);   // points per thread, the largest radix
+        f.nst_vec = zm::radix_schedule(pl->g.vec, fept, f.rad_vec);
+        f.nst_m = zm::radix_schedule(pl->g.m, fept, f.rad_m);
         B->fields.push_back(f);
         B->field_plan.push_back(pi);
         B->elems += (n[i] * n[i] + 1) & ~int64_t{1};

@@ -109,8 +109,9 @@ ZM_DEV void run_subfft(cpx<T> *s, const Geom &g, int n, int logn, const int *rad
     else stockham_stage<RR, EPT, COLM, DIR, false, T>(s, g, n, logn, Ns, nthr, tid, twN);
         if (R == 2) { ZM_STAGE(2) }
         else if (R == 4) { ZM_STAGE(4) }
-        else if (R == 8) { ZM_STAGE(8) }
-        else {
+        else if (R == 8) {
+            if constexpr (EPT >= 8) { ZM_STAGE(8) }
+        } else {
             if constexpr (EPT >= 16) { ZM_STAGE(16) }
         }
 #undef ZM_STAGE
