@@ -320,7 +320,8 @@ int zm_batch_inverse(zm_batch batch, const void *in, void *out, void *work, int 
  * the k = 0 mode set to 0, then (when `residual` is not NULL)
  * residual = Lap_h(phi) - rhs with the 5-point Laplacian / h^2.  The forward y pass, the
  * division and the inverse y pass are fused (the spectrum is never stored).  `work` holds
- * one batch buffer of scratch; rhs is kept.
+ * one batch buffer of scratch; rhs is kept.  phi is the same, bit for bit, with and without
+ * the residual.
  */
 int zm_batch_poisson(zm_batch batch, const void *rhs, void *phi, void *residual, void *work,
                      double length, void *stream);

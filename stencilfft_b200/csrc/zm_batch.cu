@@ -2,16 +2,18 @@
 //
 // A batch is a list of fields, each with its own (N, B, P) reference layout, packed one
 // after the other in every batch buffer.  One call is one cooperative launch of
-// batch_kernel: a grid of exactly the CTAs that fit on the device at once walks a short
+// a persistent kernel: a grid of exactly the CTAs that fit on the device at once walks a short
 // program of steps (an axis pass over all fields, a fused y pass, a stencil, a
 // generator ...), with a grid barrier between steps.  Inside a pass step the work items
 // are tiles of TL lines of one field, TL * N = a fixed number of points per tile, so the
-// same CTA shape serves every N; a tile's field comes from a binary search over the
-// fields' first tile numbers.  Three kernels hold the tile code: batch_axis_kernel on the
-// axis pass sized by N alone (zm_batch_axis.cuh); batch_exact_kernel (zm_batch_exact.cu) for
-// the complex64 Poisson call with a residual, which keeps the rounding of the VEC x M split
-// (see zm_batch_poisson); and batch_kernel on that split (zm_tile.cuh) for those calls where
-// a field's VEC is 1 or above 16, and for fields below N = 64.
+// same CTA shape serves every N; a tile's field comes from a table, or in batch_kernel from a
+// binary search over the fields' first tile numbers.  Three kernels hold the tile code:
+// batch_axis_kernel on the axis pass sized by N alone (zm_batch_axis.cuh);
+// batch_exact_kernel (zm_batch_exact.cu) for the complex64 Poisson call, which keeps the
+// rounding of the VEC x M split (see zm_batch_poisson); and batch_kernel on that split
+// (zm_tile.cuh) for a whole batch where one field does not fit the others' tiles: complex64
+// Poisson calls with a field of VEC = 1 or above 16 (its compile-time VEC = 4 tiles serve
+// that field's neighbours), and complex128 batches with a field of N = 32.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,8 +44,7 @@ ZM_DEV int field_of_tile(const BatchField *fields, int nfields, int64_t tile) {
 }
 
 // Both sub-transforms of a tile: compile-time-sized stages (LMC = log2 M) for the
-// complex64 tiles with VEC = 4 and P = 2 or 4 (the layout the B autotuner picks for the
-// batch sizes, B = N / 8 at P = 2), or the runtime-sized stages (LMC = 0) for every other
+// complex64 tiles with VEC = 4 and P = 2 or 4 (B = N / 8 at P = 2), or the runtime-sized stages (LMC = 0) for every other
 // shape.  (LMC > 0: the column sub-transform only; the row stage runs fused with the
 // vector-side sweep, tile_load_rows_v4 / tile_rows_store_v4)
 template <typename T, int EPT, bool INV, int LM, typename SW>
@@ -700,10 +701,11 @@ int zm_batch_poisson(zm_batch batch, const void *rhs, void *phi, void *residual,
     }
     // The complex64 residual is a difference of nearly equal terms: it amplifies phi's
     // rounding by about 8 N / (2 pi)^2 (2e-5 of the residual at N = 256, 2e-4 at 2048), so
-    // another order of the transforms' operations is another residual field.  Those calls
+    // another order of the transforms' operations is another residual field.  Complex64 calls
     // keep the rounding of the VEC x M split, on its own tiles (zm_batch_exact.cu) or, for
-    // fields that these do not hold, on batch_kernel.
-    return launch(batch, s, ns, stream, batch->dtype == ZM_C128 || !residual ? zm::TILES_AXIS : zm::TILES_EXACT);
+    // fields that these do not hold, on batch_kernel; without a residual as well, so that phi
+    // does not depend on whether the residual is asked for.
+    return launch(batch, s, ns, stream, batch->dtype == ZM_C128 ? zm::TILES_AXIS : zm::TILES_EXACT);
 }
 
 int zm_batch_status(zm_batch batch, int *device_error) {

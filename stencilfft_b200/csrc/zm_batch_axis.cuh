@@ -2,10 +2,11 @@
 //
 // A tile is 4096 points: TL = 4096 / N lines of one field, 256 threads of 16 points, so one
 // CTA shape serves every N from 64 to 4096 and every (P, B); the field's layout is its two
-// weight tables in global memory.  The fused Poisson y step keeps the spectrum of a tile in
-// registers: the last digit's forward DFT, the division and the same digit's inverse DFT
-// are one stage, so it costs five barriers and four shared-memory round trips instead of
-// the two transforms' eight and seven.
+// weight tables in global memory.  The fused Poisson y step (complex128; complex64 calls run
+// the tiles of zm_batch_exact.cu) keeps the spectrum of a tile in registers: the last
+// digit's forward DFT, the division and the same digit's inverse DFT are one stage, so it
+// costs five barriers and four shared-memory round trips instead of the two transforms'
+// eight and seven.
 #pragma once
 
 #include "zm_axis.cuh"
@@ -31,8 +32,9 @@ template <int LN, int LE> ZM_DEV int axis_low_freq(int iu) {
 // The last digit of a y tile: forward DFT, times -1 / (a^2 |k|^2) (k = 0 -> 0), inverse DFT.
 // Line l0 + t holds the x frequency ct(cid L + lp(p)) of its row p of rank column cid
 // (reciprocal_to_global, utils.h:265-268).
-template <typename T, int LN, int LTL, int LP, int LE>
-ZM_DEV void poisson_stage(cpx<T> *S, const Geom &g, int64_t l0, double a, int tid) {
+template <int LN, int LTL, int LP, int LE>
+ZM_DEV void poisson_stage(cpx<double> *S, const Geom &g, int64_t l0, double a, int tid) {
+    using T = double;
     using A = AxisPass<T, LN, LTL, LP, LE, false>;
     constexpr int NST = A::NST, lr = axis_lr(LN, LE, NST - 1), R = 1 << lr, N = 1 << LN;
     const T a2 = (T)(a * a);
@@ -51,9 +53,7 @@ ZM_DEV void poisson_stage(cpx<T> *S, const Geom &g, int64_t l0, double a, int ti
         for (int r = 0; r < R; r++) {
             const int k = k0 + (r << (LN - lr)), sy = r >= R / 2 ? k - N : k;
             const int ksq = sx2 + sy * sy;
-            T f;
-            if constexpr (sizeof(T) == 4) f = ksq == 0 ? 0.f : -__frcp_rn(a2 * (float)ksq);
-            else f = ksq == 0 ? 0.0 : -1.0 / (a2 * (double)ksq);
+            const T f = ksq == 0 ? 0.0 : -1.0 / (a2 * (double)ksq);
             x[r] = {x[r].x * f, x[r].y * f};
         }
         dft<R, 1, T, A::COMP>(x);
@@ -81,11 +81,11 @@ __device__ __noinline__ void batch_axis_tile(int op, cpx<T> *S, const cpx<T> *in
         AF::run(S, in + la.a_base, out + la.f_base, m, tb, tid, false, T(1), T(0));
     } else if (op == ATILE_INV) {
         AI::run(S, in + la.f_base, out + la.a_base, m, tb, tid, scale != T(1), scale, T(0));
-    } else {
+    } else if constexpr (sizeof(T) == 8) {
         AF::load_vec(S, in + la.a_base, m, tid);
         AF::template inner_stages<0>(S, tb, tid);
         __syncthreads();
-        poisson_stage<T, LN, LTL, LP, LE>(S, g, l0, a, tid);
+        poisson_stage<LN, LTL, LP, LE>(S, g, l0, a, tid);
         __syncthreads();
         AI::template inner_stages<AI::NST - 2>(S, tb, tid);
         AI::store_vec(S, out + la.a_base, m, tid, false, T(1), T(0));
