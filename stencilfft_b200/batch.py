@@ -92,7 +92,8 @@ class Batch:
         return v.value
 
     def barrier_probe(self, missing: int, stream=None) -> None:
-        """Launch the grid-barrier probe (missing = 1: the barrier times out by design)."""
+        """Launch the grid-barrier probe on this batch's kernels (missing = 1: the barriers time
+        out by design)."""
         check(lib().zm_batch_barrier_probe(self._h, int(missing), _stream_ptr(stream)), "zm_batch_barrier_probe")
 
     @staticmethod

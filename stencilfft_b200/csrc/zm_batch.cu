@@ -731,7 +731,9 @@ int zm_batch_barrier_probe(zm_batch batch, int missing, void *stream) {
     zm::BatchStep s[2] = {};
     s[0].op = zm::BOP_NOP;
     s[1].op = zm::BOP_NOP;
-    return launch(batch, s, 2, stream, zm::TILES_SPLIT, (unsigned)missing);
+    // the kernels that this batch's calls launch: one, and for complex64 the Poisson call's
+    if ((rc = launch(batch, s, 2, stream, zm::TILES_AXIS, (unsigned)missing)) || batch->dtype == ZM_C128) return rc;
+    return launch(batch, s, 2, stream, zm::TILES_EXACT, (unsigned)missing);
 }
 
 int zm_batch_autotune_b(int64_t n, int64_t p, int dtype, int count, int reps, int64_t *best_b, float *best_ms) {

@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_exact_kernel(const Bat
     for (int st = 0; st < bp.nsteps; st++) {
         if (st > 0 && !grid_barrier(bp.bar, gridDim.x + bp.missing, bp.abort, bp.err, &s_ok)) return;
         const int op = bp.step[st].op;
+        if (op == BOP_NOP) continue;
         const BatchStep &S = bp.step[st];
         const int ntiles = (int)bp.tiles, hop = walks_back(bp, st) ? -(int)gridDim.x : (int)gridDim.x;
         int tile = hop < 0 ? ntiles - 1 - (int)blockIdx.x : (int)blockIdx.x;
