@@ -498,6 +498,19 @@ def run_profile_case(args):
         print(json.dumps({"profile_case": {"ops": "batch", "fields": len(sizes), "dtype": args.profile_dtype,
                                            "elems": bt.total}}))
         return
+    if args.profile_ops == "batchfft":
+        # forward and inverse transforms of 16 fields of 1024^2 (P = 2, B = N / 8), two calls each
+        from stencilfft_b200 import Batch
+        bt = Batch([1024] * 16, [128] * 16, [2] * 16, dtype=args.profile_dtype)
+        x, spec, work = bt.empty(), bt.empty(), bt.empty()
+        bt.fill(x, abi.ZM_FIELD_GAUSSIAN, 100)
+        for _ in range(2):
+            bt.forward_fft(x, spec)
+            bt.inverse_fft(spec, x, work=work)
+        torch.cuda.synchronize()
+        print(json.dumps({"profile_case": {"ops": "batchfft", "fields": 16, "dtype": args.profile_dtype,
+                                           "elems": bt.total}}))
+        return
     if args.profile_ops == "layout":
         # natural -> interleaved converter, a reciprocal-space pointwise operator and the
         # natural <-> reciprocal converters, N = 8192
@@ -580,8 +593,8 @@ def main():
                     help="run the small profiling case only (for ncu captures)")
     ap.add_argument("--profile-n", type=int, default=8192)
     ap.add_argument("--profile-dtype", default="c64")
-    ap.add_argument("--profile-ops", choices=["all", "fwd", "inv", "stencils", "lap3d", "fft3d", "batch", "layout"],
-                    default="all")
+    ap.add_argument("--profile-ops", choices=["all", "fwd", "inv", "stencils", "lap3d", "fft3d", "batch", "batchfft",
+                                                  "layout"], default="all")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.profile_case:

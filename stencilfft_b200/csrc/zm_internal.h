@@ -19,9 +19,10 @@ int max_dyn_smem();
 int report_error(int code, const char *fmt, ...);
 
 // A launch that may be scheduled while the stream's previous kernel drains (programmatic
-// stream serialization); the kernel calls overlap_wait (zm_common.cuh).  It hides a launch's
-// latency behind the kernel before it: forward + inverse + Laplacian 2D N = 1024 c128 57.5 ->
-// 49 us, c64 39 -> 31, 3D N = 64 c64 45 -> 37; filter pipeline 2D N = 2048 c64 118 -> 97.
+// stream serialization); the kernel calls overlap_wait and reads fields by coherent loads
+// (ld_field, zm_common.cuh).  It hides a launch's latency behind the kernel before it:
+// forward + inverse + Laplacian 2D N = 1024 c128 57.5 -> 49 us, c64 39 -> 31, 3D N = 64 c64
+// 45 -> 37; filter pipeline 2D N = 2048 c64 118 -> 97.
 template <typename... K, typename... A>
 cudaError_t launch_overlapped(void (*kern)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
                               A &&...args) {
